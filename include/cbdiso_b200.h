@@ -465,6 +465,11 @@ int cbdiso_b200_reduce(
  * out[4i+3] = PLM slope of (a, b, a + b) with theta 1.5. */
 int cbdiso_b200_eval_primitives(long n, const double *a, const double *b, double *out, void *stream);
 
+/* Test hook: the quotient and roots the kernels use in place of the CUDA
+ * operators: out[3i] = a / b, out[3i+1] = sqrt |b|, out[3i+2] = a / sqrt |b|
+ * with both operations rounded. */
+int cbdiso_b200_eval_roots(long n, const double *a, const double *b, double *out, void *stream);
+
 /* ------------------------------------------------------------------------
  * 3. the gamma-law sibling, cbdgam_2d (sailfish/solvers/cbdgam_2d.c)
  *
@@ -604,7 +609,8 @@ void cbdgam_b200_abi_sizes(size_t out[2]);
 
 /* Test hook (no counterpart in the reference): the correctly rounded powers
  * the gamma-law kernels use, on device arrays of n elements: out[8i + 0..6]
- * = x^3, x^-2, x^-3, x^4, x^-1.5, (1 + x)^RN(-1/3), exp(-x); out[8i + 7] = 0. */
+ * = x^3, x^-2, x^-3, x^4, x^-1.5, (1 + x)^RN(-1/3), exp(-x), and in out[8i + 7]
+ * r^-3 of the rounded root r of the rounded x^2 + 1e-12. */
 int cbdgam_b200_eval_powers(long n, const double *x, double *out, void *stream);
 
 #ifdef __cplusplus

@@ -133,6 +133,8 @@ def _declare(lib):
     lib.cbdiso_b200_stage_record.restype = c_int
     lib.cbdiso_b200_eval_primitives.argtypes = [ctypes.c_long, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.cbdiso_b200_eval_primitives.restype = c_int
+    lib.cbdiso_b200_eval_roots.argtypes = [ctypes.c_long, c_void_p, c_void_p, c_void_p, c_void_p]
+    lib.cbdiso_b200_eval_roots.restype = c_int
     lib.cbdiso_b200_stepper_bytes.argtypes = []
     lib.cbdiso_b200_stepper_bytes.restype = c_size_t
     lib.cbdiso_b200_stepper_init.argtypes = [POINTER(Grid), POINTER(Orbit), c_int, c_double, c_double, c_double,
@@ -246,6 +248,7 @@ def exported_symbols():
         "cbdiso_b200_status_string", "cbdiso_b200_version", "cbdiso_b200_scratch_bytes", "cbdiso_b200_fill_guards",
         "cbdiso_b200_advance_stage", "cbdiso_b200_reduce", "cbdiso_b200_abi_sizes",
         "cbdiso_b200_stage_record_bytes", "cbdiso_b200_stage_record", "cbdiso_b200_eval_primitives",
+        "cbdiso_b200_eval_roots",
         "cbdiso_b200_advance_stage_noalloc", "cbdiso_b200_face_cache_bytes", "cbdiso_b200_advance_stage_cached",
         "cbdiso_b200_stepper_bytes", "cbdiso_b200_stepper_init",
         "cbdiso_b200_step_prologue", "cbdiso_b200_batch_disk_bytes", "cbdiso_b200_batch_disk_record",

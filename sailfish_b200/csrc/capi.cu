@@ -537,4 +537,13 @@ int cbdiso_b200_eval_primitives(long n, const double *a, const double *b, double
     return status_of(launch_primitives(n, a, b, out, static_cast<cudaStream_t>(stream)));
 }
 
+int cbdiso_b200_eval_roots(long n, const double *a, const double *b, double *out, void *stream)
+{
+    if (n < 0 || (n > 0 && (!a || !b || !out)))
+        return CBD_ERR_ARGUMENT;
+    if (n == 0)
+        return CBD_OK;
+    return status_of(launch_roots(n, a, b, out, static_cast<cudaStream_t>(stream)));
+}
+
 }  // extern "C"

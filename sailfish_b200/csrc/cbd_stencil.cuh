@@ -116,7 +116,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y)
 template <bool FAST>
 __device__ __forceinline__ double div_rn(double a, double b)
 {
-    return div_by<FAST>(a, b, __drcp_rn(b));
+    return div_by<FAST>(a, b, FAST ? crm::recip_near(b) : crm::recip_rn(b));
 }
 
 // correctly rounded powers (cr_math.cuh)
@@ -128,27 +128,23 @@ template <bool FAST>
 __device__ __forceinline__ double inv_pow15(double s2)
 {
     if (FAST) {
-        const double rs = rsqrt(s2);
+        const double rs = crm::rsqrt_near(s2);
         return rs * rs * rs;
     }
-    return (s2 > 0.0 && s2 < 1e300) ? pow_m15_rn(s2) : pow(s2, -1.5);
+    return pow_m15_rn(s2);
 }
 
-// Generalised minmod, cbdiso_2d.c:23-29. Returns exactly the value of
-// 0.25 |sgn a + sgn b| (sgn a + sgn c) min(|a|, |b|, |c|), signed zeros
-// included, with the sign logic done on integer sign bits.
+// Generalised minmod, cbdiso_2d.c:23-29: the value of
+// 0.25 |sgn a + sgn b| (sgn a + sgn c) min(|a|, |b|, |c|) with a, b, c =
+// theta (y0 - yl), (yr - yl) / 2, theta (yr - y0), up to the sign of a zero.
+// Rounding is monotonic, so theta min(|dl|, |dr|) is min(|a|, |c|), and where
+// dl and dr are nonzero with one sign yr - yl has it too: one test of the two
+// differences' sign bits decides.
 __device__ __forceinline__ double limited_slope(double yl, double y0, double yr, double theta)
 {
-    double a = (y0 - yl) * theta;
-    double b = (yr - yl) * 0.5;
-    double c = (yr - y0) * theta;
-    double m = lesser(fabs(a), lesser(fabs(b), fabs(c)));
-    unsigned sa = (unsigned)__double2hiint(a) >> 31;
-    unsigned sb = (unsigned)__double2hiint(b) >> 31;
-    unsigned sc = (unsigned)__double2hiint(c) >> 31;
-    if ((sa == sb) & (sa == sc))
-        return sa ? -m : m;
-    return (sa & sc & (sa ^ sb)) ? -0.0 : 0.0;
+    const double dl = y0 - yl, dr = yr - y0;
+    const double m = lesser(0.5 * fabs(yr - yl), theta * lesser(fabs(dl), fabs(dr)));
+    return (__double2hiint(dl) ^ __double2hiint(dr)) < 0 ? 0.0 : copysign(m, dl);
 }
 
 // softened potential of the masses with positive mass, cbdiso_2d.c:70-95
@@ -164,7 +160,7 @@ __device__ __forceinline__ double potential(const MassDev *m, double x, double y
         double dy = y - m[p].y;
         double r2 = dx * dx + dy * dy;
         double s2 = r2 + m[p].soft2;
-        term[p] = FAST ? m[p].mass * rsqrt(s2) : div_rn<false>(m[p].mass, sqrt(s2));
+        term[p] = FAST ? m[p].mass * crm::rsqrt_near(s2) : crm::over_sqrt_rn(m[p].mass, s2);
     }
     double phi = 0.0;
 #pragma unroll
@@ -205,11 +201,14 @@ __device__ __forceinline__ void hlle(const double *pl, const double *pr, double 
     const double fr1 = DIR == 0 ? vr * ur1 + gr : vr * ur1;
     const double fr2 = DIR == 1 ? vr * ur2 + gr : vr * ur2;
     if (!CS_GIVEN)
-        cs = sqrt(cs2);
-    const double am = lesser(0.0, lesser(vl - cs, vr - cs));
-    const double ap = greater(0.0, greater(vl + cs, vr + cs));
+        cs = crm::sqrt_rn(cs2);
+    // rounding is monotonic: min(vl - cs, vr - cs) is min(vl, vr) - cs
+    const bool left_less = vl < vr;
+    const double sm = (left_less ? vl : vr) - cs, sp = (left_less ? vr : vl) + cs;
+    const double am = __double2hiint(sm) < 0 ? sm : 0.0;
+    const double ap = __double2hiint(sp) < 0 ? 0.0 : sp;
     const double den = ap - am;
-    const double y = FAST ? 1.0 / den : __drcp_rn(den);
+    const double y = FAST ? crm::recip_near(den) : crm::recip_rn(den);
     if (FAST) {
         const double apam = ap * am;
         f[0] = (fl0 * ap - fr0 * am - (ul0 - ur0) * apam) * y;
@@ -286,7 +285,7 @@ __device__ __forceinline__ void mass_source(const MassDev &m, double x, double y
     }
     if (!SINK || m.sink_rate == 0.0 || m.sink_model < 1 || m.sink_model > 3 || !(r2 < m.sink_hi2))
         return;
-    const double dr = sqrt(r2);
+    const double dr = crm::sqrt_rn(r2);
     if (!(dr < m.sink_r4))
         return;
     // CUDA's exp here: a correctly rounded one (crm::exp_rn) changed no zone
@@ -307,7 +306,7 @@ __device__ __forceinline__ void mass_source(const MassDev &m, double x, double y
         break;
     case 2: {
         const double d = dr + 1e-12;
-        const double yd = FAST ? 1.0 / d : __drcp_rn(d);
+        const double yd = FAST ? crm::recip_near(d) : crm::recip_rn(d);
         const double ex = div_by<FAST>(dx, d, yd);
         const double ey = div_by<FAST>(dy, d, yd);
         const double dvr = (p[1] - m.vx) * ex + (p[2] - m.vy) * ey;
@@ -334,11 +333,11 @@ __device__ __forceinline__ void buffer_source(const Consts &k, const StageDev &s
     const double r2 = x * x + y * y;
     if (!(r2 > k.buf_lo2))
         return;
-    const double rc = sqrt(r2);
+    const double rc = crm::sqrt_rn(r2);
     if (!(rc > k.buf_onset))
         return;
-    const double yr = FAST ? 1.0 / rc : __drcp_rn(rc);
-    const double vk = sqrt(div_by<FAST>(st.buffer_mass, rc, yr));
+    const double yr = FAST ? crm::recip_near(rc) : crm::recip_rn(rc);
+    const double vk = crm::sqrt_rn(div_by<FAST>(st.buffer_mass, rc, yr));
     const double t1 = k.buf_sigma * div_by<FAST>(-y, rc, yr) * vk;
     const double t2 = k.buf_sigma * div_by<FAST>(+x, rc, yr) * vk;
     const double rate = div_by<FAST>(st.buffer_k * (rc - k.buf_onset), k.buf_span, k.inv_buf_span);
@@ -353,7 +352,7 @@ __device__ __forceinline__ void cons_to_prim(const double *u, double *p, const C
 {
     const double rho = greater(u[0], k.rho_min);
     p[0] = rho;
-    const double y = FAST ? 1.0 / rho : __drcp_rn(rho);
+    const double y = FAST ? crm::recip_near(rho) : crm::recip_rn(rho);
     p[1] = copysign(lesser(fabs(div_by<FAST>(u[1], rho, y)), k.vmax), u[1]);
     p[2] = copysign(lesser(fabs(div_by<FAST>(u[2], rho, y)), k.vmax), u[2]);
 }
@@ -361,7 +360,7 @@ __device__ __forceinline__ void cons_to_prim(const double *u, double *p, const C
 // max |v +- cs| over both directions, cbdiso_2d.c:340-350
 __device__ __forceinline__ double max_wavespeed(const double *p, double cs2)
 {
-    const double cs = sqrt(cs2);
+    const double cs = crm::sqrt_rn(cs2);
     const double ax = greater(fabs(p[1] - cs), fabs(p[1] + cs));
     const double ay = greater(fabs(p[2] - cs), fabs(p[2] + cs));
     return greater(ax, ay);
@@ -379,12 +378,8 @@ __device__ __forceinline__ void end_rates(const MassDev *e, int need, double x, 
     for (int q = 0; q < 2; ++q) {
         rg[q][0] = rg[q][1] = rg[q][2] = 0.0;
         ra[q][0] = ra[q][1] = ra[q][2] = 0.0;
-        if (need & (1 << q)) {
-            // the gravity rates only enter sums whose own rounding (their
-            // summation order) is far above an ulp per zone: rsqrt-based
-            // arithmetic, not the correctly rounded power
-            mass_source<true, true, false>(e[q], x, y, 1.0, p, rg[q]);
-        }
+        if (need & (1 << q))
+            mass_source<FAST, true, false>(e[q], x, y, 1.0, p, rg[q]);
         if (need & (4 << q))
             mass_source<FAST, false, true>(e[q], x, y, 1.0, p, ra[q]);
     }
@@ -1288,11 +1283,11 @@ __device__ __forceinline__ void face_cache_fill_point(const Consts &k, const Mas
     const double yc = k.yl + ((double)j + 0.5) * k.dy;
     if (j < nj) {
         const double cs2 = sound_speed2<FAST>(k, m, xf, yc);
-        cache_store(c.xf + 2 * ((size_t)i * nj + j), cs2, sqrt(cs2));
+        cache_store(c.xf + 2 * ((size_t)i * nj + j), cs2, crm::sqrt_rn(cs2));
     }
     if (i < ni) {
         const double cs2 = sound_speed2<FAST>(k, m, xc, yf);
-        cache_store(c.yf + 2 * ((size_t)i * (nj + 1) + j), cs2, sqrt(cs2));
+        cache_store(c.yf + 2 * ((size_t)i * (nj + 1) + j), cs2, crm::sqrt_rn(cs2));
     }
     if (i < ni && j < nj) {
         double g[2] = {0.0, 0.0};

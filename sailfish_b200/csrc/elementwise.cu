@@ -111,6 +111,16 @@ __global__ void primitives_kernel(long n, const double *a, const double *b, doub
     }
 }
 
+// quotients and roots without CUDA's slow paths: a / b, sqrt |b|, a / sqrt |b|
+__global__ void roots_kernel(long n, const double *a, const double *b, double *out)
+{
+    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        out[3 * i] = div_rn<false>(a[i], b[i]);
+        out[3 * i + 1] = crm::sqrt_rn(fabs(b[i]));
+        out[3 * i + 2] = crm::over_sqrt_rn(a[i], fabs(b[i]));
+    }
+}
+
 inline int blocks_for(long n, int bs, int cap)
 {
     long b = (n + bs - 1) / bs;
@@ -151,6 +161,12 @@ cudaError_t launch_fill_guards(int ni, int nj, double *p, cudaStream_t s)
 cudaError_t launch_primitives(long n, const double *a, const double *b, double *out, cudaStream_t s)
 {
     primitives_kernel<<<blocks_for(n, 256, 148 * 16), 256, 0, s>>>(n, a, b, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_roots(long n, const double *a, const double *b, double *out, cudaStream_t s)
+{
+    roots_kernel<<<blocks_for(n, 256, 148 * 16), 256, 0, s>>>(n, a, b, out);
     return cudaGetLastError();
 }
 

@@ -53,8 +53,9 @@ struct Consts {
     double theta, gamma, alpha, cooling, mach_ceiling, vmax, rho_floor, p_floor;
     int constant_softening;
     int buffer_on;
-    double buf_sigma, buf_pressure, buf_rate, buf_outer, buf_width;
-    double buf_onset_m3;  // pow(buf_outer - buf_width, -3.0), glibc's on the host
+    // the buffer: Sigma, internal energy and onset radius of its target, the span
+    // of its ramp, a squared radius surely inside the onset, reciprocals
+    double buf_sigma, buf_energy, buf_onset, buf_span, buf_lo2, inv_buf_sigma, inv_buf_span;
     double mach_m2;       // pow(mach_ceiling, -2.0), glibc's on the host
     double inv_dx, inv_dy, gm1, inv_gm1, inv_gamma;  // RN(1 / dx), ..., gamma - 1, RN(1 / (gamma - 1)), RN(1 / gamma)
 };
@@ -62,6 +63,7 @@ struct Consts {
 struct Stage {
     Mass m[2];
     double buf_mass, a, dt;
+    double buf_k;  // driving rate times the orbital frequency at the onset radius
     int massless;  // both masses have zero mass: every scale height is 1
     int write_guards;
     int un_from_primitive;  // u_n = cons(primitive_n) in-kernel (else: a conserved array)
@@ -78,6 +80,8 @@ using crm::inv_cube_rn;
 using crm::inv_pow15_rn;
 using crm::inv_square_rn;
 using crm::pow_m13_rn;
+using crm::recip_rn;
+using crm::sqrt_rn;
 
 __device__ __forceinline__ double lesser(double a, double b) { return a < b ? a : b; }
 __device__ __forceinline__ double greater(double a, double b) { return a > b ? a : b; }
@@ -85,40 +89,44 @@ __device__ __forceinline__ double sign_of(double x) { return copysign(1.0, x); }
 __device__ __forceinline__ size_t at(int i, int j, int nj) { return ((size_t)(i + NG) * (nj + 2 * NG) + (j + NG)) * NF; }
 
 // cbdgam_2d.c:27-33: 0.25 |sgn a + sgn b| (sgn a + sgn c) min(|a|, |b|, |c|),
-// returned exactly (signed zeros included) with the sign logic done on the
-// sign bits: it is m, -m, +0 or -0.
+// up to the sign of a zero: theta min(|dl|, |dr|) is min(|a|, |c|) because
+// rounding is monotonic, and where dl and dr are nonzero with one sign yr - yl
+// has it too.
 __device__ __forceinline__ double slope(double yl, double y0, double yr, double theta)
 {
-    const double a = (y0 - yl) * theta;
-    const double b = (yr - yl) * 0.5;
-    const double c = (yr - y0) * theta;
-    const double m = lesser(fabs(a), lesser(fabs(b), fabs(c)));
-    const unsigned sa = (unsigned)__double2hiint(a) >> 31;
-    const unsigned sb = (unsigned)__double2hiint(b) >> 31;
-    const unsigned sc = (unsigned)__double2hiint(c) >> 31;
-    if ((sa == sb) & (sa == sc))
-        return sa ? -m : m;
-    return (sa & sc & (sa ^ sb)) ? -0.0 : 0.0;
+    const double dl = y0 - yl, dr = yr - y0;
+    const double m = lesser(0.5 * fabs(yr - yl), theta * lesser(fabs(dl), fabs(dr)));
+    return (__double2hiint(dl) ^ __double2hiint(dr)) < 0 ? 0.0 : copysign(m, dl);
 }
 
 template <class V>
 __device__ __forceinline__ double cs2_of(double gamma, const V &p) { return p[3] / p[0] * gamma; }
 
+// a / b rounded to nearest from y = RN(1 / b): the remainder a - q b of
+// q = RN(a y) is exact under FMA and one correction rounds to RN(a / b)
+__device__ __forceinline__ double div_by(double a, double b, double y)
+{
+    const double q = a * y;
+    return fma(fma(-q, b, a), y, q);
+}
+
+__device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, recip_rn(b)); }
+
 // cbdgam_2d.c:238-276
-__device__ __forceinline__ void buffer_source(const Consts &k, double buf_mass, double x, double y, double dt,
+__device__ __forceinline__ void buffer_source(const Consts &k, const Stage &st, double x, double y, double dt,
                                               double *u)
 {
-    if (!k.buffer_on)
+    const double r2 = x * x + y * y;
+    if (!k.buffer_on || !(r2 > k.buf_lo2))
         return;
-    const double rc = sqrt(x * x + y * y);
-    const double onset = k.buf_outer - k.buf_width;
-    if (rc > onset) {
-        const double pf = k.buf_sigma * sqrt(buf_mass / rc);
-        const double px = pf * (-y / rc), py = pf * (x / rc);
-        const double ek = 0.5 * (px * px + py * py) / k.buf_sigma;
-        const double target[NF] = {k.buf_sigma, px, py, k.buf_pressure / (k.gamma - 1.0) + ek};
-        const double omega = sqrt(buf_mass * k.buf_onset_m3);  // pow(onset, -3.0), from the host
-        const double rate = k.buf_rate * omega * (rc - onset) / (k.buf_outer - onset);
+    const double rc = sqrt_rn(r2);
+    if (rc > k.buf_onset) {
+        const double yr = recip_rn(rc);
+        const double pf = k.buf_sigma * sqrt_rn(div_by(st.buf_mass, rc, yr));
+        const double px = pf * div_by(-y, rc, yr), py = pf * div_by(x, rc, yr);
+        const double ek = div_by(0.5 * (px * px + py * py), k.buf_sigma, k.inv_buf_sigma);
+        const double target[NF] = {k.buf_sigma, px, py, k.buf_energy + ek};
+        const double rate = div_by(st.buf_k * (rc - k.buf_onset), k.buf_span, k.inv_buf_span);
 #pragma unroll
         for (int q = 0; q < NF; ++q)
             u[q] -= (u[q] - target[q]) * rate * dt;
@@ -140,7 +148,7 @@ __device__ __forceinline__ void prim_to_cons(const V &p, double *u, double gamma
 template <class V>
 __device__ __forceinline__ double max_wavespeed(const V &p, double cs2)
 {
-    const double cs = sqrt(cs2);
+    const double cs = sqrt_rn(cs2);
     const double ax = greater(fabs(p[1] - cs), fabs(p[1] + cs));
     const double ay = greater(fabs(p[2] - cs), fabs(p[2] + cs));
     return greater(ax, ay);
@@ -160,14 +168,6 @@ __device__ __forceinline__ double max_wavespeed(const V &p, double cs2)
 // reciprocal rounded to nearest and a Markstein correction, which returns
 // the correctly rounded quotient.
 // ---------------------------------------------------------------------------
-
-// a / b rounded to nearest from y = RN(1 / b): the remainder a - q b of
-// q = RN(a y) is exact under FMA and one correction rounds to RN(a / b)
-__device__ __forceinline__ double div_by(double a, double b, double y)
-{
-    const double q = a * y;
-    return fma(fma(-q, b, a), y, q);
-}
 
 constexpr int ZI = TI + 2, ZJ = TJ + 2;  // zones with shared quantities: the tile and a ring of one
 // per-zone quantities: x and y slopes, p / Sigma, sound speed, sqrt(p / Sigma), strain xx, xy, yy
@@ -189,11 +189,10 @@ __device__ __forceinline__ double root_w2(const Mass *m, double x, double y)
     for (int k = 0; k < 2; ++k) {
         if (m[k].mass > 0.0) {
             const double dx = x - m[k].x, dy = y - m[k].y;
-            const double r = sqrt(dx * dx + dy * dy + 1e-12);
-            w2 += m[k].mass * inv_cube_rn(r);
+            w2 += m[k].mass * crm::inv_cube_of_sqrt_rn(dx * dx + dy * dy + 1e-12);
         }
     }
-    return sqrt(w2);
+    return sqrt_rn(w2);
 }
 
 // cbdgam_2d.c:347-362 with the constant divisor gamma - 1
@@ -219,9 +218,12 @@ __device__ __forceinline__ void hlle_fast(const Consts &k, const double *pl, con
                            vl * (ul[3] + pl[3])};
     const double fr[NF] = {vr * ur[0], vr * ur[1] + pr[3] * (double)(DIR == 0), vr * ur[2] + pr[3] * (double)(DIR == 1),
                            vr * (ur[3] + pr[3])};
-    const double am = lesser(0.0, lesser(vl - cs, vr - cs));
-    const double ap = greater(0.0, greater(vl + cs, vr + cs));
-    const double den = ap - am, y = __drcp_rn(den);
+    // rounding is monotonic: min(vl - cs, vr - cs) is min(vl, vr) - cs
+    const bool left_less = vl < vr;
+    const double sm = (left_less ? vl : vr) - cs, sp = (left_less ? vr : vl) + cs;
+    const double am = __double2hiint(sm) < 0 ? sm : 0.0;
+    const double ap = __double2hiint(sp) < 0 ? 0.0 : sp;
+    const double den = ap - am, y = recip_rn(den);
 #pragma unroll
     for (int q = 0; q < NF; ++q)
         f[q] = div_by(fl[q] * ap - fr[q] * am - (ul[q] - ur[q]) * ap * am, den, y);
@@ -235,10 +237,28 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
                                             const double *g_in = nullptr, double *g_out = nullptr)
 {
     const double sigma = p[0];
-    const double eps = div_by(T, gm1, inv_gm1);
     const double dx = x - m.x, dy = y - m.y;
     const double r2 = dx * dx + dy * dy;
-    const double dr = sqrt(r2);
+    // Beyond four sink radii (with a margin far above the square root's
+    // rounding) the sink rate is zero and the softening, if it follows the
+    // disk height, is half of it: only gravity's terms are left, the others
+    // being exact zeros.
+    const double far2 = 16.0 * (m.radius * m.radius);
+    if (r2 > far2 * (1.0 + 1e-10)) {
+        const double soft = constant_softening ? m.soft : 0.5 * h;
+        const double g = g_in ? *g_in : crm::pow_m15_rn(r2 + soft * soft);
+        if (g_out)
+            *g_out = g;
+        const double fnum = m.model >= 1 && m.model <= 3 ? sigma * m.mass * g : 0.0;
+        const double fx = -fnum * dx, fy = -fnum * dy;
+        du[0] = 0.0;
+        du[1] = dt * fx;
+        du[2] = dt * fy;
+        du[3] = dt * (fx * p[1] + fy * p[2]);
+        return;
+    }
+    const double eps = div_by(T, gm1, inv_gm1);
+    const double dr = sqrt_rn(r2);
     const double rs = m.radius;
     double soft;
     if (constant_softening) {
@@ -252,7 +272,7 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
     }
     const double rate = (dr < 4.0 * rs) ? m.rate * exp_rn(-fourth_rn(dr / rs)) : 0.0;
     // the gravity factor: from the face cache (constant softening), or computed
-    const double g = g_in ? *g_in : inv_pow15_rn(r2 + soft * soft);
+    const double g = g_in ? *g_in : crm::pow_m15_rn(r2 + soft * soft);
     if (g_out)
         *g_out = g;
     const double fnum = sigma * m.mass * g;
@@ -265,7 +285,7 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
         du[2] = dt * mdot * p[2] + dt * fy;
         du[3] = dt * (mdot * eps + 0.5 * mdot * (vx * vx + vy * vy)) + dt * (fx * vx + fy * vy);
     } else if (m.model == 2) {
-        const double den = dr + 1e-12, yd = __drcp_rn(den);
+        const double den = dr + 1e-12, yd = recip_rn(den);
         const double ex = div_by(dx, den, yd), ey = div_by(dy, den, yd);
         const double dvr = (vx - m.vx) * ex + (vy - m.vy) * ey;
         const double wx = dvr * ex + m.vx, wy = dvr * ey + m.vy;
@@ -302,7 +322,7 @@ __device__ __forceinline__ void cooling_fast(const Consts &k, double dt, const V
 // cbdgam_2d.c:319-345 with one reciprocal of Sigma
 __device__ __forceinline__ void c2p_fast(const Consts &k, const double *u, double *p)
 {
-    const double y = __drcp_rn(u[0]);
+    const double y = recip_rn(u[0]);
     double pres = greater(k.p_floor, (u[3] - div_by(0.5 * (u[1] * u[1] + u[2] * u[2]), u[0], y)) * k.gm1);
     double vx = sign_of(u[1]) * lesser(fabs(div_by(u[1], u[0], y)), k.vmax);
     double vy = sign_of(u[2]) * lesser(fabs(div_by(u[2], u[0], y)), k.vmax);
@@ -454,10 +474,10 @@ __device__ __forceinline__ void stage_phase1(const Consts &k, const Stage &st, S
             sm.z[Q_GX + q][a][b] = gx[q];
             sm.z[Q_GY + q][a][b] = gy[q];
         }
-        const double T = sm.prim[3][a + 1][b + 1] / sm.prim[0][a + 1][b + 1];
+        const double T = div_rn(sm.prim[3][a + 1][b + 1], sm.prim[0][a + 1][b + 1]);
         sm.z[Q_T][a][b] = T;
-        sm.z[Q_CS][a][b] = sqrt(T * k.gamma);  // sqrt(cs2), cs2 = p / Sigma * gamma (cbdgam_2d.c:231-236)
-        sm.z[Q_SQ][a][b] = sqrt(T);
+        sm.z[Q_CS][a][b] = sqrt_rn(T * k.gamma);  // sqrt(cs2), cs2 = p / Sigma * gamma (cbdgam_2d.c:231-236)
+        sm.z[Q_SQ][a][b] = sqrt_rn(T);
         // strain (cbdgam_2d.c:278-294): (4/3 gx_vx) / dx - (2/3 gy_vy) / dy, ...
         sm.z[Q_SXX][a][b] = div_by(4.0 / 3.0 * gx[1], k.dx, k.inv_dx) - div_by(2.0 / 3.0 * gy[2], k.dy, k.inv_dy);
         sm.z[Q_SXY][a][b] = div_by(gx[2], k.dx, k.inv_dx) + div_by(gy[1], k.dy, k.inv_dy);
@@ -523,13 +543,13 @@ __device__ __forceinline__ void stage_phase2(const Consts &k, const Stage &st, c
     } else if (!st.massless) {
         wc = root_w2(st.m, xc, yc);
     }
-    const double hc = st.massless ? 1.0 : Z(0, 0, Q_SQ) / wc;
+    const double hc = st.massless ? 1.0 : div_rn(Z(0, 0, Q_SQ), wc);
 
     if (k.alpha > 0.0) {
-        const double hw = st.massless ? 1.0 : Z(-1, 0, Q_SQ) / sm.fx[ty][tx];
-        const double he = st.massless ? 1.0 : Z(1, 0, Q_SQ) / sm.fx[ty + 1][tx];
-        const double hs = st.massless ? 1.0 : Z(0, -1, Q_SQ) / sm.fy[ty][tx];
-        const double hn = st.massless ? 1.0 : Z(0, 1, Q_SQ) / sm.fy[ty][tx + 1];
+        const double hw = st.massless ? 1.0 : div_rn(Z(-1, 0, Q_SQ), sm.fx[ty][tx]);
+        const double he = st.massless ? 1.0 : div_rn(Z(1, 0, Q_SQ), sm.fx[ty + 1][tx]);
+        const double hs = st.massless ? 1.0 : div_rn(Z(0, -1, Q_SQ), sm.fy[ty][tx]);
+        const double hn = st.massless ? 1.0 : div_rn(Z(0, 1, Q_SQ), sm.fy[ty][tx + 1]);
         const double nuc = k.alpha * hc * Z(0, 0, Q_CS);
         const double nuw = k.alpha * hw * Z(-1, 0, Q_CS), nue = k.alpha * he * Z(1, 0, Q_CS);
         const double nus = k.alpha * hs * Z(0, -1, Q_CS), nun = k.alpha * hn * Z(0, 1, Q_CS);
@@ -564,7 +584,7 @@ __device__ __forceinline__ void stage_phase2(const Consts &k, const Stage &st, c
     const double T = Z(0, 0, Q_T);
     double u[NF];
     p2c_fast(k, c, u);
-    buffer_source(k, st.buf_mass, xc, yc, dt, u);
+    buffer_source(k, st, xc, yc, dt, u);
 #pragma unroll
     for (int m = 0; m < 2; ++m) {
         double du[NF];
@@ -657,7 +677,7 @@ __global__ void __launch_bounds__(NT, STAGE_MIN_BLOCKS) stage_kernel(Consts k, S
                     dst[q] = out[q];
             }
         if (ws_max)
-            ws = max_nan(ws, max_wavespeed(out, cs2_of(k.gamma, out)));
+            ws = max_nan(ws, max_wavespeed(out, div_rn(out[3], out[0]) * k.gamma));
     }
     if (ws_max) {  // uniform over the block
 #pragma unroll
@@ -705,7 +725,7 @@ __global__ void __launch_bounds__(128) cache_fill_kernel(Consts k, Stage st, dou
                 for (int p = 0; p < 2; ++p) {
                     const double dx = xc - st.m[p].x, dy = yc - st.m[p].y;
                     const double r2 = dx * dx + dy * dy;
-                    g[p] = inv_pow15_rn(r2 + st.m[p].soft * st.m[p].soft);
+                    g[p] = crm::pow_m15_rn(r2 + st.m[p].soft * st.m[p].soft);
                 }
                 const size_t z = (size_t)i * nj + j;
                 *reinterpret_cast<double2 *>(cv.zp + 2 * z) = make_double2(root_w2(st.m, xc, yc), g[0]);
@@ -902,7 +922,7 @@ __global__ void eval_powers_kernel(long n, const double *x, double *out)
         o[4] = inv_pow15_rn(v);
         o[5] = pow_m13_rn(1.0 + v);
         o[6] = exp_rn(-v);
-        o[7] = 0.0;
+        o[7] = crm::inv_cube_of_sqrt_rn(v * v + 1e-12);
     }
 }
 
@@ -936,11 +956,12 @@ Consts consts_of(const cbdgam_grid_t *g)
     k.constant_softening = g->constant_softening;
     k.buffer_on = g->buffer_is_enabled;
     k.buf_sigma = g->buffer_surface_density;
-    k.buf_pressure = g->buffer_surface_pressure;
-    k.buf_rate = g->buffer_driving_rate;
-    k.buf_outer = g->buffer_outer_radius;
-    k.buf_width = g->buffer_onset_width;
-    k.buf_onset_m3 = std::pow(g->buffer_outer_radius - g->buffer_onset_width, -3.0);
+    k.buf_energy = g->buffer_surface_pressure / (k.gamma - 1.0);
+    k.buf_onset = g->buffer_outer_radius - g->buffer_onset_width;
+    k.buf_span = g->buffer_outer_radius - k.buf_onset;
+    k.buf_lo2 = k.buf_onset > 0.0 ? k.buf_onset * k.buf_onset * (1.0 - 1e-10) : -1.0;
+    k.inv_buf_sigma = 1.0 / k.buf_sigma;
+    k.inv_buf_span = 1.0 / k.buf_span;
     k.mach_m2 = std::pow(g->mach_ceiling, -2.0);
     k.inv_dx = 1.0 / k.dx;
     k.inv_dy = 1.0 / k.dy;
@@ -948,6 +969,12 @@ Consts consts_of(const cbdgam_grid_t *g)
     k.inv_gm1 = 1.0 / k.gm1;
     k.inv_gamma = 1.0 / k.gamma;
     return k;
+}
+
+// cbdgam_2d.c:266-267 on the host, with the C library's pow
+double buffer_k(double driving_rate, double central_mass, double outer_radius, double onset_width)
+{
+    return driving_rate * std::sqrt(central_mass * std::pow(outer_radius - onset_width, -3.0));
 }
 
 Mass mass_of(const cbd_mass_t &m)
@@ -1100,6 +1127,7 @@ int cbdgam_2d_advance_rk(int ni, int nj, double xl, double xr, double yl, double
     st.m[0] = mass_args(x1, y1, vx1, vy1, mass1, softening_length1, sink_rate1, sink_radius1, sink_model1);
     st.m[1] = mass_args(x2, y2, vx2, vy2, mass2, softening_length2, sink_rate2, sink_radius2, sink_model2);
     st.buf_mass = buffer_central_mass;
+    st.buf_k = buffer_k(buffer_driving_rate, buffer_central_mass, buffer_outer_radius, buffer_onset_width);
     st.a = a;
     st.dt = dt;
     st.write_guards = 0;
@@ -1166,6 +1194,8 @@ int advance_stage(const cbdgam_grid_t *grid, const cbdgam_stage_t *stage, const 
     st.m[0] = mass_of(stage->mass[0]);
     st.m[1] = mass_of(stage->mass[1]);
     st.buf_mass = stage->buffer_central_mass;
+    st.buf_k = buffer_k(grid->buffer_driving_rate, stage->buffer_central_mass, grid->buffer_outer_radius,
+                        grid->buffer_onset_width);
     st.a = stage->a;
     st.dt = stage->dt;
     st.write_guards = 1;
