@@ -40,17 +40,41 @@ struct BatchArgs {
     double *fcache;      // face-cache arena (disk d's cache at disks[d].cache_offset), or null
 };
 
+// the disk that tile u belongs to
+__device__ __forceinline__ int disk_of_unit(const BatchArgs &a, int u)
+{
+    int lo = 0, hi = a.num_disks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (a.disks[mid].unit_begin <= u)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    return lo;
+}
+
+// disk d's constants and stage record into shared memory, a word per thread
+template <int BJ>
+__device__ __forceinline__ void load_disk(const BatchArgs &a, int d, Consts &k, StageDev &st)
+{
+    const double *src = reinterpret_cast<const double *>(&a.disks[d].k);
+    double *dst = reinterpret_cast<double *>(&k);
+    for (int w = threadIdx.x; w < (int)(sizeof(Consts) / sizeof(double)); w += BJ)
+        dst[w] = src[w];
+    load_record<BJ>(st, st, &a.records[(size_t)d * a.num_stages + a.stage]);
+}
+
 // ROLE (ROLE_*) is what the launch does with each disk's face cache: a writer
 // stores into the caches of the disks that have one; a reader requires one
 // for every disk (the batch's fill kernel ran before it), skips the tiles of
 // a disk without one, and the disk's first tile records the key.
-template <int BJ, int MINB, int PREC, int ROLE = ROLE_NONE, bool EPI = true, bool RATES = false>
+template <int BJ, int MINB, int PREC, int ROLE = ROLE_NONE>
 __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs a)
 {
     constexpr bool FAST = PREC == CBD_PRECISION_FAST;
     __shared__ Consts k;
     __shared__ StageDev st;
-    __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
     __shared__ int s_unit, s_disk;
     const int t = threadIdx.x;
 
@@ -58,41 +82,19 @@ __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs
         if (t == 0) {
             const int u = (int)atomicAdd(&a.counters[0], 1u);
             s_unit = u;
-            if (u < a.total_units) {
-                int lo = 0, hi = a.num_disks - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) / 2;
-                    if (a.disks[mid].unit_begin <= u)
-                        lo = mid;
-                    else
-                        hi = mid - 1;
-                }
-                s_disk = lo;
-            }
+            if (u < a.total_units)
+                s_disk = disk_of_unit(a, u);
         }
         __syncthreads();
         const int u = s_unit;
         if (u >= a.total_units)
             break;
         const DiskDev &D = a.disks[s_disk];
-        {
-            const double *src = reinterpret_cast<const double *>(&D.k);
-            double *dst = reinterpret_cast<double *>(&k);
-            for (int w = t; w < (int)(sizeof(Consts) / sizeof(double)); w += BJ)
-                dst[w] = src[w];
-            const double *rs = reinterpret_cast<const double *>(&a.records[(size_t)s_disk * a.num_stages + a.stage]);
-            double *rd = reinterpret_cast<double *>(&st);
-            for (int w = t; w < (int)(sizeof(StageDev) / sizeof(double)); w += BJ)
-                rd[w] = rs[w];
-        }
+        load_disk<BJ>(a, s_disk, k, st);
         __syncthreads();
         if (t == 0) {
             k.un_kind = a.un ? 1 : 0;
             k.write_guards = 1;
-            if (!a.epilogue) {
-                k.want_ws = 0;
-                k.num_diag = 0;
-            }
         }
         __syncthreads();
         const int local = u - D.unit_begin;
@@ -107,42 +109,22 @@ __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs
         sa.result = nullptr;
         const bool cached = ROLE != ROLE_NONE && a.fcache && D.cache_offset >= 0;
         sa.fcache = cached ? a.fcache + D.cache_offset : nullptr;
-        double acc[PARTIAL_STRIDE];
-#pragma unroll
-        for (int v = 0; v < PARTIAL_STRIDE; ++v)
-            acc[v] = 0.0;
         const int c0 = strip * D.strip_width, r0 = seg * k.rows_per_cta;
         if (st.halt) {
-            // the disk's stepper stopped: no march, zero partials
+            // the disk's stepper stopped: no march
         } else if (ROLE == ROLE_WRITER) {
             // the same answer in every thread; the disk's first tile writes the key
             const bool store = cached && cache_write_check<PREC>(k, st, sa.fcache, t == 0 && u == D.unit_begin);
-            march_tile<BJ, FAST, CACHE_WRITE, EPI, false, false, RATES>(k, st, sa, c0, D.strip_width, r0, acc, store);
+            march_tile<BJ, FAST, CACHE_WRITE, false>(k, st, sa, c0, D.strip_width, r0, store);
         } else if (ROLE == ROLE_READER) {
             if (cached) {
-                march_tile<BJ, FAST, CACHE_READ, EPI, false, false, RATES>(k, st, sa, c0, D.strip_width, r0, acc);
+                march_tile<BJ, FAST, CACHE_READ, false>(k, st, sa, c0, D.strip_width, r0);
                 // the fill kernel ran before this launch; no tile reads the key
                 if (t == 0 && u == D.unit_begin)
                     cache_write_key<PREC>(k, st, sa.fcache);
             }
         } else {
-            march_tile<BJ, FAST, CACHE_NONE, EPI, false, false, RATES>(k, st, sa, c0, D.strip_width, r0, acc);
-        }
-        if (EPI) {
-            double red[PARTIAL_STRIDE];
-            block_reduce<BJ>(acc, sred, red);
-            // a disk whose diagnostics the rates-only kernel cannot evaluate
-            // (a wrong epilogue form from the caller): NaN sums, not wrong ones
-            if (RATES && !k.rates_only) {
-#pragma unroll
-                for (int v = 1; v < PARTIAL_STRIDE; ++v)
-                    red[v] = __longlong_as_double(0x7ff8000000000000LL);
-            }
-            if (t == 0) {
-#pragma unroll
-                for (int v = 0; v < PARTIAL_STRIDE; ++v)
-                    a.partials[(size_t)u * PARTIAL_STRIDE + v] = red[v];
-            }
+            march_tile<BJ, FAST, CACHE_NONE, false>(k, st, sa, c0, D.strip_width, r0);
         }
         __syncthreads();
     }
@@ -169,17 +151,10 @@ __global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ) batched_fill_
     __shared__ int s_disk, fill;
     for (int u = blockIdx.x; u < a.total_units; u += gridDim.x) {
         if (threadIdx.x == 0) {
-            int lo = 0, hi = a.num_disks - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) / 2;
-                if (a.disks[mid].unit_begin <= u)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            s_disk = lo;
-            const DiskDev &D = a.disks[lo];
-            st = a.records[(size_t)lo * a.num_stages + a.stage];
+            const int d = disk_of_unit(a, u);
+            s_disk = d;
+            const DiskDev &D = a.disks[d];
+            st = a.records[(size_t)d * a.num_stages + a.stage];
             fill = D.cache_offset >= 0 && !st.halt &&
                    !cache_key_matches<PREC>(D.k, st, a.fcache + D.cache_offset);
         }
@@ -197,6 +172,55 @@ __global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ) batched_fill_
     }
 }
 
+// The epilogue of every disk's tiles after the step's last stage: CTA u
+// reduces tile u exactly as the single grid's epilogue kernel does and leaves
+// its partials for batched_finalize. CACHED: the stage before was a writer,
+// whose gravity factors serve when its masses are the end-of-step masses.
+template <int BJ, int PREC, bool RATES>
+__global__ void __launch_bounds__(BJ, epi_warps(RATES) * 32 / BJ)
+    batched_epilogue_kernel(const BatchArgs a, const bool cached)
+{
+    constexpr bool FAST = PREC == CBD_PRECISION_FAST;
+    __shared__ Consts k;
+    __shared__ StageDev st;
+    __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
+    __shared__ int s_disk;
+    const int u = blockIdx.x, t = threadIdx.x;
+    if (t == 0)
+        s_disk = disk_of_unit(a, u);
+    __syncthreads();
+    load_disk<BJ>(a, s_disk, k, st);
+    __syncthreads();
+    const DiskDev &D = a.disks[s_disk];
+    double acc[PARTIAL_STRIDE];
+#pragma unroll
+    for (int v = 0; v < PARTIAL_STRIDE; ++v)
+        acc[v] = 0.0;
+    // a disk whose stepper stopped: zero partials
+    if (!st.halt) {
+        const int local = u - D.unit_begin;
+        const double *grav = nullptr;
+        if (cached && a.fcache && D.cache_offset >= 0 && same_cached_inputs(st))
+            grav = cache_arrays(a.fcache + D.cache_offset, k.ni, k.nj).grav;
+        epilogue_tile<BJ, FAST, RATES>(k, st, a.pwr + D.offset, grav, (local % D.strips) * D.strip_width, D.strip_width,
+                                   (local / D.strips) * k.rows_per_cta, acc);
+    }
+    double red[PARTIAL_STRIDE];
+    block_reduce<BJ, RATES>(acc, sred, red);
+    // a disk whose diagnostics the rates-only kernel cannot evaluate (a wrong
+    // epilogue form from the caller): NaN sums, not wrong ones
+    if (RATES && !k.rates_only) {
+#pragma unroll
+        for (int v = 1; v < PARTIAL_STRIDE; ++v)
+            red[v] = __longlong_as_double(0x7ff8000000000000LL);
+    }
+    if (t == 0) {
+#pragma unroll
+        for (int v = 0; v < PARTIAL_STRIDE; ++v)
+            a.partials[(size_t)u * PARTIAL_STRIDE + v] = red[v];
+    }
+}
+
 cudaError_t launch_batched_exact(const BatchArgs &a, int ctas, int role, cudaStream_t s);
 cudaError_t launch_batched_fma(const BatchArgs &a, int ctas, int role, cudaStream_t s);
 cudaError_t launch_batched_fast(const BatchArgs &a, int ctas, int role, cudaStream_t s);
@@ -208,31 +232,20 @@ cudaError_t launch_batched(const BatchArgs &a, int ctas, int role, cudaStream_t 
 {
     switch (role) {
     case ROLE_WRITER:
-        if (a.epilogue == 2)
-            batched_stage_kernel<128, 6, PREC, ROLE_WRITER, true, true><<<ctas, 128, 0, s>>>(a);
-        else if (a.epilogue)
-            batched_stage_kernel<128, 6, PREC, ROLE_WRITER, true><<<ctas, 128, 0, s>>>(a);
-        else
-            batched_stage_kernel<128, 6, PREC, ROLE_WRITER, false><<<ctas, 128, 0, s>>>(a);
+        batched_stage_kernel<128, 6, PREC, ROLE_WRITER><<<ctas, 128, 0, s>>>(a);
         break;
     case ROLE_READER:
         batched_fill_kernel<128, PREC><<<a.total_units < 148 * 8 ? a.total_units : 148 * 8, 128, 0, s>>>(a);
-        if (a.epilogue == 2)
-            batched_stage_kernel<128, 6, PREC, ROLE_READER, true, true><<<ctas, 128, 0, s>>>(a);
-        else if (a.epilogue)
-            batched_stage_kernel<128, 6, PREC, ROLE_READER, true><<<ctas, 128, 0, s>>>(a);
-        else
-            batched_stage_kernel<128, 6, PREC, ROLE_READER, false><<<ctas, 128, 0, s>>>(a);
+        batched_stage_kernel<128, 6, PREC, ROLE_READER><<<ctas, 128, 0, s>>>(a);
         break;
     default:
-        if (a.epilogue == 2)
-            batched_stage_kernel<128, 6, PREC, ROLE_NONE, true, true><<<ctas, 128, 0, s>>>(a);
-        else if (a.epilogue)
-            batched_stage_kernel<128, 6, PREC, ROLE_NONE, true><<<ctas, 128, 0, s>>>(a);
-        else
-            batched_stage_kernel<128, 6, PREC, ROLE_NONE, false><<<ctas, 128, 0, s>>>(a);
+        batched_stage_kernel<128, 6, PREC, ROLE_NONE><<<ctas, 128, 0, s>>>(a);
         break;
     }
+    if (a.epilogue == 2)
+        batched_epilogue_kernel<128, PREC, true><<<a.total_units, 128, 0, s>>>(a, role == ROLE_WRITER);
+    else if (a.epilogue)
+        batched_epilogue_kernel<128, PREC, false><<<a.total_units, 128, 0, s>>>(a, role == ROLE_WRITER);
     return cudaGetLastError();
 }
 

@@ -370,71 +370,88 @@ __device__ __forceinline__ double max_wavespeed(const double *p, double cs2)
 // reference's on/off switches (cbdiso_2d.py:105-137, cbdiso_2d.c:626-664):
 // rg[p] with gravity only, ra[p] with accretion only, each (mdot, fx, fy).
 // `need` selects which are evaluated (bit p: rg[p], bit 2 + p: ra[p]).
+// `g`: the masses' gravity factors at the zone, when the caller has them.
 template <bool FAST>
-__device__ __forceinline__ void end_rates(const MassDev *e, int need, double x, double y, const double *p,
-                                          double (&rg)[2][3], double (&ra)[2][3])
+__device__ __forceinline__ void end_gravity(const MassDev *e, int need, double x, double y, const double *p,
+                                            double (&rg)[2][3], const double *g = nullptr)
 {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         rg[q][0] = rg[q][1] = rg[q][2] = 0.0;
-        ra[q][0] = ra[q][1] = ra[q][2] = 0.0;
         if (need & (1 << q))
-            mass_source<FAST, true, false>(e[q], x, y, 1.0, p, rg[q]);
+            mass_source<FAST, true, false>(e[q], x, y, 1.0, p, rg[q], g ? g + q : nullptr);
+    }
+}
+
+template <bool FAST>
+__device__ __forceinline__ void end_accretion(const MassDev *e, int need, double x, double y, const double *p,
+                                              double (&ra)[2][3])
+{
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        ra[q][0] = ra[q][1] = ra[q][2] = 0.0;
         if (need & (4 << q))
             mass_source<FAST, false, true>(e[q], x, y, 1.0, p, ra[q]);
     }
 }
 
+// whether the zone centre lies in the reach of a mass whose accretion rates
+// are needed; elsewhere those rates are zero
+__device__ __forceinline__ bool near_sinks(const MassDev *e, int need, double x, double y)
+{
+    bool near = false;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const double dx = x - e[q].x, dy = y - e[q].y;
+        near |= (need & (4 << q)) && dx * dx + dy * dy < e[q].sink_hi2;
+    }
+    return near;
+}
+
+// Per-zone value of a source-rate diagnostic (mdot, fx, fy, torque, power) of
+// the masses' rates r, with weight w.
+__device__ __forceinline__ double rate_value(const cbd_diag_t &d, const MassDev *e, double x, double y,
+                                             const double (&r)[2][3], double w)
+{
+    double f[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        f[c] = d.which_mass == 3 ? r[0][c] + r[1][c] : (d.which_mass == 2 ? r[1][c] : r[0][c]);
+    if (d.quantity == CBD_Q_MDOT)
+        return f[0] * w;
+    if (d.quantity == CBD_Q_FX)
+        return f[1] * w;
+    if (d.quantity == CBD_Q_FY)
+        return f[2] * w;
+    if (d.quantity == CBD_Q_TORQUE)
+        return x * (f[2] * w) - y * (f[1] * w);
+    const MassDev &mv = e[d.which_mass == 2 ? 1 : 0];
+    return mv.vx * (f[1] * w) + mv.vy * (f[2] * w);
+}
+
 // Per-zone value of one diagnostic (cbdiso_2d.py:383-471): out = (re, im).
-// RATES: the caller knows that d is a source rate (mdot, fx, fy, torque,
-// power) without a radial cut, so only that code is compiled (w = 1 then,
-// the same values).
-template <bool FAST, bool RATES = false>
 __device__ __forceinline__ void diag_value(const cbd_diag_t &d, const MassDev *e, double x, double y,
                                            const double *p, const double (&rg)[2][3], const double (&ra)[2][3],
                                            double *out)
 {
     double w = 1.0, r = 0.0;
-    const bool polar = !RATES && (d.quantity == CBD_Q_SIGMA_M1 || d.quantity == CBD_Q_ECCENTRICITY_VECTOR);
-    if (!RATES && (d.has_cut || polar)) {
+    const bool polar = d.quantity == CBD_Q_SIGMA_M1 || d.quantity == CBD_Q_ECCENTRICITY_VECTOR;
+    if (d.has_cut || polar) {
         r = sqrt(x * x + y * y);
         if (d.has_cut)
             w = ((d.r0 < r) & (r < d.r1)) ? 1.0 : 0.0;
     }
     out[0] = 0.0;
     out[1] = 0.0;
-    switch (RATES ? CBD_Q_MDOT : d.quantity) {
+    switch (d.quantity) {
     case CBD_Q_MDOT:
     case CBD_Q_FX:
     case CBD_Q_FY:
     case CBD_Q_TORQUE:
-    case CBD_Q_POWER: {
+    case CBD_Q_POWER:
         // the reference takes the accretion rates when both flags are set
-        const bool acc = d.accretion != 0;
-        double r1[3], r2[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            r1[c] = acc ? ra[0][c] : rg[0][c];
-            r2[c] = acc ? ra[1][c] : rg[1][c];
-        }
-        double f[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            f[c] = d.which_mass == 3 ? r1[c] + r2[c] : (d.which_mass == 2 ? r2[c] : r1[c]);
-        if (d.quantity == CBD_Q_MDOT)
-            out[0] = f[0] * w;
-        else if (d.quantity == CBD_Q_FX)
-            out[0] = f[1] * w;
-        else if (d.quantity == CBD_Q_FY)
-            out[0] = f[2] * w;
-        else if (d.quantity == CBD_Q_TORQUE)
-            out[0] = x * (f[2] * w) - y * (f[1] * w);
-        else {
-            const MassDev &mv = e[d.which_mass == 2 ? 1 : 0];
-            out[0] = mv.vx * (f[1] * w) + mv.vy * (f[2] * w);
-        }
+        out[0] = d.accretion ? rate_value(d, e, x, y, ra, w) : rate_value(d, e, x, y, rg, w);
         break;
-    }
     case CBD_Q_SIGMA_M1:
         out[0] = p[0] * w * (x / r);
         out[1] = p[0] * w * (y / r);
@@ -460,28 +477,57 @@ __device__ __forceinline__ void diag_value(const cbd_diag_t &d, const MassDev *e
     }
 }
 
-// The end-of-step quantities of one zone, accumulated into acc: slot 0 the
-// CFL wavespeed maximum, slots 1 + 2d, 2 + 2d the diagnostics (RATES: all of
-// them source rates without a radial cut, k.rates_only).
+// The diagnostics of one zone, added into acc: slots 1 + 2d, 2 + 2d (RATES:
+// all of them source rates without a radial cut, k.rates_only).
 template <bool FAST, bool RATES = false>
+__device__ __forceinline__ void accumulate_sums(const Consts &k, const MassDev *e, double x, double y,
+                                                const double *p, double (&acc)[PARTIAL_STRIDE],
+                                                const double *g = nullptr)
+{
+    if (k.num_diag == 0)
+        return;
+    double rg[2][3], ra[2][3];
+    if (RATES) {
+        // the accretion terms are zero outside the sinks' reach, where adding
+        // them changes no sum
+        if (k.need_rates & 3) {
+            end_gravity<FAST>(e, k.need_rates, x, y, p, rg, g);
+#pragma unroll
+            for (int d = 0; d < MAX_FUSED; ++d)
+                if (d < k.num_diag && !k.diag[d].accretion)
+                    acc[1 + 2 * d] += rate_value(k.diag[d], e, x, y, rg, 1.0);
+        }
+        if (near_sinks(e, k.need_rates, x, y)) {
+            end_accretion<FAST>(e, k.need_rates, x, y, p, ra);
+#pragma unroll
+            for (int d = 0; d < MAX_FUSED; ++d)
+                if (d < k.num_diag && k.diag[d].accretion)
+                    acc[1 + 2 * d] += rate_value(k.diag[d], e, x, y, ra, 1.0);
+        }
+        return;
+    }
+    end_gravity<FAST>(e, k.need_rates, x, y, p, rg, g);
+    end_accretion<FAST>(e, k.need_rates, x, y, p, ra);
+#pragma unroll
+    for (int d = 0; d < MAX_FUSED; ++d) {
+        if (d < k.num_diag) {
+            double v[2];
+            diag_value(k.diag[d], e, x, y, p, rg, ra, v);
+            acc[1 + 2 * d] += v[0];
+            acc[2 + 2 * d] += v[1];
+        }
+    }
+}
+
+// The end-of-step quantities of one zone, accumulated into acc: slot 0 the
+// CFL wavespeed maximum, the others the diagnostics.
+template <bool FAST>
 __device__ __forceinline__ void accumulate_zone(const Consts &k, const MassDev *e, double x, double y,
                                                 const double *p, double (&acc)[PARTIAL_STRIDE])
 {
     if (k.want_ws)
         acc[0] = max_nan(acc[0], max_wavespeed(p, sound_speed2<FAST>(k, e, x, y)));
-    if (k.num_diag > 0) {
-        double rg[2][3], ra[2][3];
-        end_rates<FAST>(e, k.need_rates, x, y, p, rg, ra);
-#pragma unroll
-        for (int d = 0; d < MAX_FUSED; ++d) {
-            if (d < k.num_diag) {
-                double v[2];
-                diag_value<FAST, RATES>(k.diag[d], e, x, y, p, rg, ra, v);
-                acc[1 + 2 * d] += v[0];
-                acc[2 + 2 * d] += v[1];
-            }
-        }
-    }
+    accumulate_sums<FAST>(k, e, x, y, p, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -491,7 +537,8 @@ __device__ __forceinline__ void accumulate_zone(const Consts &k, const MassDev *
 // Reduces PARTIAL_STRIDE per-thread values over the block in a fixed order:
 // slot 0 by max, the others by sum. Thread 0 receives the results in `out`.
 // All indices are compile-time constants so the values stay in registers.
-template <int BJ>
+// REAL: the diagnostics' imaginary slots are zero and left out.
+template <int BJ, bool REAL = false>
 __device__ __forceinline__ void block_reduce(const double (&vals)[PARTIAL_STRIDE], double *smem,
                                              double (&out)[PARTIAL_STRIDE])
 {
@@ -499,6 +546,8 @@ __device__ __forceinline__ void block_reduce(const double (&vals)[PARTIAL_STRIDE
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int v = 0; v < PARTIAL_STRIDE; ++v) {
+        if (REAL && v > 0 && v % 2 == 0)
+            continue;
         double x = vals[v];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -512,6 +561,10 @@ __device__ __forceinline__ void block_reduce(const double (&vals)[PARTIAL_STRIDE
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int v = 0; v < PARTIAL_STRIDE; ++v) {
+            if (REAL && v > 0 && v % 2 == 0) {
+                out[v] = 0.0;
+                continue;
+            }
             double x = smem[v * NW];
             for (int w = 1; w < NW; ++w)
                 x = v == 0 ? max_nan(x, smem[v * NW + w]) : x + smem[v * NW + w];
@@ -586,6 +639,19 @@ __device__ __forceinline__ void async_copy8(void *smem, const void *gmem)
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 __device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+__device__ __forceinline__ void async_copy16(void *smem, const void *gmem)
+{
+    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+// waits until at most N of this thread's most recent groups are in flight
+template <int N>
+__device__ __forceinline__ void async_wait()
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
 // ---------------------------------------------------------------------------
 // the fused stage kernel
@@ -783,18 +849,15 @@ constexpr size_t march_dynamic_smem()
 
 // One tile of the march: columns c0 .. c0 + width - 1 (width <= BJ) and rows
 // r0 .. r0 + k.rows_per_cta - 1 of one grid. `st` must live in shared memory
-// and be visible after the first barrier; epilogue values of the updated
-// zones are accumulated into `acc` when EPI (the launch has an epilogue;
-// without, its code is left out). `COP` (CACHE_*) says what the tile does
-// with args.fcache: CACHE_WRITE stores the face and gravity values if
+// and be visible after the first barrier. `COP` (CACHE_*) says what the tile
+// does with args.fcache: CACHE_WRITE stores the face and gravity values if
 // `store`, CACHE_READ loads them. ONE_SYNC marches with one barrier per row
 // (five-row ring, u_n in registers), otherwise with two (four-row ring, u_n
 // through shared memory), which needs fewer registers: the persistent
 // batched kernel keeps it. All threads of the block must call it.
-template <int BJ, bool FAST, int COP = CACHE_NONE, bool EPI = true, bool ONE_SYNC = true, bool P2 = false,
-          bool RATES = false>
+template <int BJ, bool FAST, int COP = CACHE_NONE, bool ONE_SYNC = true, bool P2 = false>
 __device__ __forceinline__ void march_tile(const Consts &k, const StageDev &st, const StageArgs &args, int c0,
-                                           int width, int r0, double (&acc)[PARTIAL_STRIDE], bool store = false)
+                                           int width, int r0, bool store = false)
 {
     constexpr int cop = COP;
     StageSmem<BJ, ONE_SYNC> &sm = stage_smem<BJ, ONE_SYNC>();
@@ -1143,9 +1206,6 @@ __device__ __forceinline__ void march_tile(const Consts &k, const StageDev &st, 
                     }
                 }
             }
-
-            if (EPI)
-                accumulate_zone<FAST, RATES>(k, st.e, xc, yc, pn, acc);
         }
 
 #pragma unroll
@@ -1161,23 +1221,28 @@ __device__ __forceinline__ void march_tile(const Consts &k, const StageDev &st, 
     __syncthreads();
 }
 
+// A launch's stage record into shared memory, a word per thread (visible
+// after the next barrier).
+template <int BJ>
+__device__ __forceinline__ void load_record(StageDev &st, const StageDev &param, const StageDev *dev)
+{
+    static_assert(sizeof(StageDev) % sizeof(double) == 0, "copied in doubles");
+    const double *src = reinterpret_cast<const double *>(dev ? dev : &param);
+    double *dst = reinterpret_cast<double *>(&st);
+    for (int w = threadIdx.x; w < (int)(sizeof(StageDev) / sizeof(double)); w += BJ)
+        dst[w] = src[w];
+}
+
 // One RK stage on one grid: CTA (x, y) marches strip x, segment y. ROLE
-// (ROLE_*) is what the launch does with args.fcache; EPI whether it has an
-// epilogue (k.want_ws or k.num_diag); P2 that k.spacing_pow2 is set (the
-// divisions by dx and dy are then the products with their exact
-// reciprocals).
-template <int BJ, int MINB, int PREC, int ROLE = ROLE_NONE, bool EPI = true, bool P2 = false>
+// (ROLE_*) is what the launch does with args.fcache; P2 that k.spacing_pow2
+// is set (the divisions by dx and dy are then the products with their exact
+// reciprocals). The epilogue is a launch of its own (stage_epilogue_kernel).
+template <int BJ, int MINB, int PREC, int ROLE = ROLE_NONE, bool P2 = false>
 __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const StageDev st_param, StageArgs args)
 {
     constexpr bool FAST = PREC == CBD_PRECISION_FAST;
     __shared__ StageDev st;
-    __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
-    if (threadIdx.x == 0)
-        st = args.stage_dev ? *args.stage_dev : st_param;
-    double acc[PARTIAL_STRIDE];
-#pragma unroll
-    for (int v = 0; v < PARTIAL_STRIDE; ++v)
-        acc[v] = 0.0;
+    load_record<BJ>(st, st_param, args.stage_dev);
     const int c0 = blockIdx.x * BJ, r0 = blockIdx.y * k.rows_per_cta;
     __syncthreads();
     if (st.halt)
@@ -1185,76 +1250,159 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
     if (ROLE == ROLE_WRITER) {
         const bool store = cache_write_check<PREC>(k, st, args.fcache,
                                                    threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0);
-        march_tile<BJ, FAST, CACHE_WRITE, EPI, true, P2>(k, st, args, c0, BJ, r0, acc, store);
+        march_tile<BJ, FAST, CACHE_WRITE, true, P2>(k, st, args, c0, BJ, r0, store);
     } else if (ROLE == ROLE_READER) {
-        march_tile<BJ, FAST, CACHE_READ, EPI, true, P2>(k, st, args, c0, BJ, r0, acc);
+        march_tile<BJ, FAST, CACHE_READ, true, P2>(k, st, args, c0, BJ, r0);
         // the fill kernel before this launch made the values valid for these
         // masses; say so for the next fill (no one reads the key meanwhile)
         if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0)
             cache_write_key<PREC>(k, st, args.fcache);
     } else {
-        march_tile<BJ, FAST, CACHE_NONE, EPI, true, P2>(k, st, args, c0, BJ, r0, acc);
-    }
-    if (EPI) {
-        double red[PARTIAL_STRIDE];
-        block_reduce<BJ>(acc, sred, red);
-        grid_finish<BJ>(red, 1 + 2 * k.num_diag, args.scratch, k.want_ws ? args.result : nullptr, args.result + 1,
-                        sred);
+        march_tile<BJ, FAST, CACHE_NONE, true, P2>(k, st, args, c0, BJ, r0);
     }
 }
 
-// resident 128-thread CTAs per SM the rates-only epilogue is built for
-constexpr int EPI_RATES_MINB = 4;
+// Relative slack of the estimated wavespeeds below. The estimate's sound
+// speed comes from the gravity factors (m g s^2 = m / s to a few ulps) and a
+// Newton step on the rsqrt seed (2^-20 measured: 3/8 (2 x 2^-20)^2 < 2^-39),
+// so it is within 2^-38 of the exact value.
+constexpr double WS_SLACK = 0x1p-36;
 
 // The epilogue of one tile after its stage has written it: thread t adds up
 // the zones of column c0 + t, rows r0 .. r0 + k.rows_per_cta - 1, of the new
-// state `p` in row order, exactly as the fused march accumulates them.
-template <bool FAST, bool RATES = false>
-__device__ __forceinline__ void epilogue_tile(const Consts &k, const StageDev &st, const double *p, int c0,
-                                              int width, int r0, double (&acc)[PARTIAL_STRIDE])
+// state `p` in row order. `grav` (or null) is a face cache's gravity array
+// holding the end-of-step masses' factors.
+//
+// The wavespeed maximum has to be exact (it sets dt), but the exact value of
+// a zone takes four correctly rounded roots and quotients. An estimate with a
+// known slack is enough to drop a zone: each thread keeps the zone of its
+// column that leads by more than the slack and evaluates it exactly at the
+// end; a zone too close to the leader (or NaN) is evaluated on the spot.
+//
+// A thread's rows come through a ring of its own in shared memory, EPI_DEPTH
+// rows deep: one row ahead in registers kept 20 KB per SM in flight, about a
+// third of what HBM needs (4096^2: 230 us a launch).
+constexpr int EPI_DEPTH = 4;
+
+template <int BJ>
+struct EpilogueSmem {
+    double2 g[EPI_DEPTH][BJ];
+    double p[EPI_DEPTH][NQ][BJ];
+};
+
+template <int BJ, bool FAST, bool RATES>
+__device__ __forceinline__ void epilogue_tile(const Consts &k, const StageDev &st, const double *p,
+                                              const double *grav, int c0, int width, int r0,
+                                              double (&acc)[PARTIAL_STRIDE])
 {
     const int t = threadIdx.x;
     const int W = min(width, k.nj - c0);
     const int r1 = min(r0 + k.rows_per_cta, k.ni);
-    if (t >= W)
+    if (t >= W || r0 >= r1)
         return;
     const int j = c0 + t;
     const size_t row_stride = (size_t)(k.nj + 2 * NG) * NQ;
     const double yc = k.yl + ((double)j + 0.5) * k.dy;
     const double *z = p + (size_t)(r0 + NG) * row_stride + (size_t)(j + NG) * NQ;
-    if (r0 >= r1)
-        return;
-    double nx[NQ] = {z[0], z[1], z[2]};
-    for (int r = r0; r < r1; ++r) {
-        const double pn[NQ] = {nx[0], nx[1], nx[2]};
-        z += row_stride;
-        if (r + 1 < r1) {
-            nx[0] = z[0];
-            nx[1] = z[1];
-            nx[2] = z[2];
+    const double *gz = grav + 2 * ((size_t)r0 * k.nj + j);
+    __shared__ EpilogueSmem<BJ> ring;
+    // the next row into slot `slot`, as one group (empty past the last row)
+    int fetched = r0;
+    auto fetch = [&](int slot) {
+        if (fetched < r1) {
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                async_copy8(&ring.p[slot][q][t], z + q);
+            if (grav)
+                async_copy16(&ring.g[slot][t], gz);
+            z += row_stride;
+            gz += 2 * (size_t)k.nj;
+            ++fetched;
         }
-        const double xc = k.xl + ((double)r + 0.5) * k.dx;
-        accumulate_zone<FAST, RATES>(k, st.e, xc, yc, pn, acc);
+        async_commit();
+    };
+#pragma unroll
+    for (int d = 0; d + 1 < EPI_DEPTH; ++d)
+        fetch(d);
+    int slot = 0;
+    double lead = -1.0, lead_v[2] = {0.0, 0.0};
+    int lead_r = r0;
+    // r = r1 is the leader's exact evaluation
+    for (int r = r0; r <= r1; ++r) {
+        double pn[NQ];
+        bool exact = false;
+        double xc = k.xl + ((double)r + 0.5) * k.dx;
+        if (r < r1) {
+            // into the slot read last; then row r has landed
+            fetch((slot + EPI_DEPTH - 1) % EPI_DEPTH);
+            async_wait<EPI_DEPTH - 1>();
+#pragma unroll
+            for (int q = 0; q < NQ; ++q)
+                pn[q] = ring.p[slot][q][t];
+            double g[2] = {0.0, 0.0};
+            if (grav) {
+                const double2 v = ring.g[slot][t];
+                g[0] = v.x;
+                g[1] = v.y;
+            }
+            slot = (slot + 1) % EPI_DEPTH;
+            double c = 0.0;
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double dx = xc - st.e[q].x, dy = yc - st.e[q].y;
+                const double s2 = dx * dx + dy * dy + st.e[q].soft2;
+                if (!grav) {
+                    const double gq = inv_pow15<FAST>(s2);
+                    g[q] = st.e[q].mass != 0.0 ? gq : 0.0;
+                }
+                const double term = st.e[q].mass * (g[q] * s2);
+                c = st.e[q].mass > 0.0 ? c + term : c;
+            }
+            if (k.want_ws) {
+                const double c2 = k.eos == 2 ? c * k.inv_mach2 : (k.eos == 1 ? k.cs2 : 1.0);
+                const double y = crm::rsqrt_seed(c2), h = c2 * y;
+                const double est = greater(fabs(pn[1]), fabs(pn[2])) + fma(0.5 * h, fma(-h, y, 1.0), h);
+                if (est > lead * (1.0 + WS_SLACK)) {
+                    lead = est;
+                    lead_v[0] = pn[1];
+                    lead_v[1] = pn[2];
+                    lead_r = r;
+                } else {
+                    exact = !(est < lead * (1.0 - WS_SLACK));
+                }
+            }
+            accumulate_sums<FAST, RATES>(k, st.e, xc, yc, pn, acc, g);
+        } else if (lead >= 0.0) {
+            exact = true;
+            pn[0] = 0.0;
+            pn[1] = lead_v[0];
+            pn[2] = lead_v[1];
+            xc = k.xl + ((double)lead_r + 0.5) * k.dx;
+        }
+        if (exact)
+            acc[0] = max_nan(acc[0], max_wavespeed(pn, sound_speed2<FAST>(k, st.e, xc, yc)));
     }
 }
 
-// A stage's epilogue as its own launch, after a stage kernel launched
-// without it (EPI = false) on the same grid: the same CTA tiles, per-thread
-// order, block tree and CTA order, so the same bits as the fused epilogue.
-// Reading the new state back (24 B per zone) costs less than carrying the
-// epilogue's registers and code through the stencil's march. (As two
-// launches, the wavespeed maximum and the diagnostic sums each with its own
-// register budget, it measured slower.) RATES: the form for k.rates_only,
-// with fewer registers.
-template <int BJ, int PREC, bool RATES = false>
-__global__ void __launch_bounds__(BJ, (RATES ? EPI_RATES_MINB : 4) * 128 / BJ)
+// resident warps per SM the epilogue kernels are built for: 24 (80 registers,
+// no spills) for the source rates, 4096^2 190 -> 160 us a launch against 16;
+// the generic form would spill at 80 registers
+constexpr int epi_warps(bool rates) { return rates ? 24 : 16; }
+
+// A stage's epilogue as its own launch after the stage kernel, on the same
+// grid of tiles: per-thread row order, block tree, then CTA order. Reading the
+// new state back (24 B per zone, and 16 B of gravity factors that a writer
+// stage just stored) costs less than carrying the epilogue's registers and
+// code through the stencil's march. args.fcache: a cache whose gravity
+// factors are the stage masses'; used when those are the end-of-step masses.
+template <int BJ, int PREC, bool RATES>
+__global__ void __launch_bounds__(BJ, epi_warps(RATES) * 32 / BJ)
     stage_epilogue_kernel(const Consts k, const StageDev st_param, StageArgs args)
 {
     constexpr bool FAST = PREC == CBD_PRECISION_FAST;
     __shared__ StageDev st;
     __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
-    if (threadIdx.x == 0)
-        st = args.stage_dev ? *args.stage_dev : st_param;
+    load_record<BJ>(st, st_param, args.stage_dev);
     __syncthreads();
     if (st.halt)
         return;
@@ -1262,9 +1410,10 @@ __global__ void __launch_bounds__(BJ, (RATES ? EPI_RATES_MINB : 4) * 128 / BJ)
 #pragma unroll
     for (int v = 0; v < PARTIAL_STRIDE; ++v)
         acc[v] = 0.0;
-    epilogue_tile<FAST, RATES>(k, st, args.pwr, blockIdx.x * BJ, BJ, blockIdx.y * k.rows_per_cta, acc);
+    const double *grav = args.fcache && same_cached_inputs(st) ? cache_arrays(args.fcache, k.ni, k.nj).grav : nullptr;
+    epilogue_tile<BJ, FAST, RATES>(k, st, args.pwr, grav, blockIdx.x * BJ, BJ, blockIdx.y * k.rows_per_cta, acc);
     double red[PARTIAL_STRIDE];
-    block_reduce<BJ>(acc, sred, red);
+    block_reduce<BJ, RATES>(acc, sred, red);
     grid_finish<BJ>(red, 1 + 2 * k.num_diag, args.scratch, k.want_ws ? args.result : nullptr, args.result + 1, sred);
 }
 

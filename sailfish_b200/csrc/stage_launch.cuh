@@ -22,7 +22,7 @@ cudaError_t prepare_stage_kernel()
     if (dev < 0 || dev >= 64)
         return cudaErrorInvalidDevice;
     if (!ready[dev]) {
-        e = cudaFuncSetAttribute(stage_kernel<BJ, MINB, PREC, ROLE, false, P2>,
+        e = cudaFuncSetAttribute(stage_kernel<BJ, MINB, PREC, ROLE, P2>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess)
             return e;
@@ -41,11 +41,9 @@ cudaError_t launch_one_p2(const LaunchShape &s, const Consts &k, const StageDev 
                                           : prepare_stage_kernel<BJ, MINB, PREC, ROLE_NONE, P2>();
     if (e != cudaSuccess)
         return e;
-    // a stage with an epilogue runs as the stage without it, then the
-    // epilogue kernel over the same tiles (the same bits as fusing them)
     switch (role) {
     case ROLE_WRITER:
-        stage_kernel<BJ, MINB, PREC, ROLE_WRITER, false, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
+        stage_kernel<BJ, MINB, PREC, ROLE_WRITER, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
         break;
     case ROLE_READER: {
         // the fill over the stage's own tiles, then the stage
@@ -53,18 +51,21 @@ cudaError_t launch_one_p2(const LaunchShape &s, const Consts &k, const StageDev 
         const int per_sm = FILL_WARPS_PER_SM * 32 / BJ;
         const int fill_ctas = tiles < 148 * per_sm ? tiles : 148 * per_sm;
         face_cache_fill_kernel<BJ, PREC><<<fill_ctas, BJ, 0, stream>>>(k, st, a.stage_dev, a.fcache, s.grid.x, tiles);
-        stage_kernel<BJ, MINB, PREC, ROLE_READER, false, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
+        stage_kernel<BJ, MINB, PREC, ROLE_READER, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
         break;
     }
     default:
-        stage_kernel<BJ, MINB, PREC, ROLE_NONE, false, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
+        stage_kernel<BJ, MINB, PREC, ROLE_NONE, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
         break;
     }
     if (k.want_ws || k.num_diag > 0) {
+        // the epilogue over the stage's tiles; a writer's cache holds its masses' factors
+        StageArgs e = a;
+        e.fcache = role == ROLE_WRITER ? a.fcache : nullptr;
         if (k.rates_only)
-            stage_epilogue_kernel<BJ, PREC, true><<<s.grid, BJ, 0, stream>>>(k, st, a);
+            stage_epilogue_kernel<BJ, PREC, true><<<s.grid, BJ, 0, stream>>>(k, st, e);
         else
-            stage_epilogue_kernel<BJ, PREC, false><<<s.grid, BJ, 0, stream>>>(k, st, a);
+            stage_epilogue_kernel<BJ, PREC, false><<<s.grid, BJ, 0, stream>>>(k, st, e);
     }
     return cudaGetLastError();
 }
