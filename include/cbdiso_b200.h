@@ -349,7 +349,7 @@ int cbdiso_b200_batched_stage(const void *disks, int num_disks, int total_units,
 
 /* cbdiso_b200_batched_stage with face caches and a role (as in
  * cbdiso_b200_advance_stage_cached: 0 none, 1 writer, 2 reader, the reader
- * preceded by a fill pass over every disk's tiles). Disk d's cache lies at face_cache + its
+ * preceded by a fill pass over the disks). Disk d's cache lies at face_cache + its
  * record's cache offset, set by cbdiso_b200_batch_disk_set_face_cache (an even
  * number of doubles); it holds cbdiso_b200_face_cache_bytes(its grid) bytes
  * with its first 256 bytes zeroed before the first use, and `face_cache` is

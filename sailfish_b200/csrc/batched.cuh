@@ -113,14 +113,14 @@ __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs
         if (st.halt) {
             // the disk's stepper stopped: no march
         } else if (ROLE == ROLE_WRITER) {
-            // the same answer in every thread; the disk's first tile writes the key
-            const bool store = cached && cache_write_check<PREC>(k, st, sa.fcache, t == 0 && u == D.unit_begin);
+            // the same answer in every thread; the block with the disk's first tile writes the key
+            const bool store = cached && cache_write_check<PREC>(k, st, sa.fcache, u == D.unit_begin);
             march_tile<BJ, FAST, CACHE_WRITE, false>(k, st, sa, c0, D.strip_width, r0, store);
         } else if (ROLE == ROLE_READER) {
             if (cached) {
                 march_tile<BJ, FAST, CACHE_READ, false>(k, st, sa, c0, D.strip_width, r0);
                 // the fill kernel ran before this launch; no tile reads the key
-                if (t == 0 && u == D.unit_begin)
+                if (u == D.unit_begin)
                     cache_write_key<PREC>(k, st, sa.fcache);
             }
         } else {
@@ -140,36 +140,27 @@ __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs
 }
 
 // The face caches of every disk valid for a reader stage (see
-// face_cache_fill_kernel): CTA b takes tiles u = b, b + gridDim.x, ... of the
-// batch's tile list (the same tiles as the stage) and fills tile u when its
-// disk has a cache whose key does not match the disk's stage masses.
+// face_cache_fill_kernel): CTA (d, b) compares disk d's key and, when it does
+// not match the disk's stage masses, fills the disk's tiles b, b + gridDim.y,
+// ... (One comparison per tile, by one thread, took 37 us for 1864 tiles of 24
+// disks.)
 template <int BJ, int PREC>
 __global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ) batched_fill_kernel(const BatchArgs a)
 {
-    constexpr bool FAST = PREC == CBD_PRECISION_FAST;
+    __shared__ Consts k;
     __shared__ StageDev st;
-    __shared__ int s_disk, fill;
-    for (int u = blockIdx.x; u < a.total_units; u += gridDim.x) {
-        if (threadIdx.x == 0) {
-            const int d = disk_of_unit(a, u);
-            s_disk = d;
-            const DiskDev &D = a.disks[d];
-            st = a.records[(size_t)d * a.num_stages + a.stage];
-            fill = D.cache_offset >= 0 && !st.halt &&
-                   !cache_key_matches<PREC>(D.k, st, a.fcache + D.cache_offset);
-        }
-        __syncthreads();
-        if (fill) {
-            const DiskDev &D = a.disks[s_disk];
-            const int local = u - D.unit_begin;
-            const int strip = local % D.strips;
-            const int seg = local / D.strips;
-            face_cache_fill_tile<BJ, FAST>(D.k, st.m, a.fcache + D.cache_offset, strip * D.strip_width,
-                                           D.strip_width, seg * D.k.rows_per_cta, D.k.rows_per_cta);
-        }
-        // the shared record is rewritten for the next tile
-        __syncthreads();
-    }
+    const DiskDev &D = a.disks[blockIdx.x];
+    if (D.cache_offset < 0)
+        return;
+    load_disk<BJ>(a, blockIdx.x, k, st);
+    __syncthreads();
+    double *fc = a.fcache + D.cache_offset;
+    if (cache_key_matches<PREC>(k, st, fc) || st.halt)
+        return;
+    for (int u = blockIdx.y; u < D.strips * D.segments; u += gridDim.y)
+        face_cache_fill_tile<BJ, PREC == CBD_PRECISION_FAST>(k, st.m, fc, (u % D.strips) * D.strip_width,
+                                                             D.strip_width, (u / D.strips) * k.rows_per_cta,
+                                                             k.rows_per_cta);
 }
 
 // The epilogue of every disk's tiles after the step's last stage: CTA u
@@ -226,7 +217,7 @@ cudaError_t launch_batched_fma(const BatchArgs &a, int ctas, int role, cudaStrea
 cudaError_t launch_batched_fast(const BatchArgs &a, int ctas, int role, cudaStream_t s);
 
 // One batched stage launch at precision PREC with a face-cache role; the
-// reader is preceded by the fill kernel.
+// reader is preceded by the fill kernel, about 6 CTAs per SM of it.
 template <int PREC>
 cudaError_t launch_batched(const BatchArgs &a, int ctas, int role, cudaStream_t s)
 {
@@ -235,7 +226,8 @@ cudaError_t launch_batched(const BatchArgs &a, int ctas, int role, cudaStream_t 
         batched_stage_kernel<128, 6, PREC, ROLE_WRITER><<<ctas, 128, 0, s>>>(a);
         break;
     case ROLE_READER:
-        batched_fill_kernel<128, PREC><<<a.total_units < 148 * 8 ? a.total_units : 148 * 8, 128, 0, s>>>(a);
+        batched_fill_kernel<128, PREC>
+            <<<dim3(a.num_disks, (148 * 6 + a.num_disks - 1) / a.num_disks), 128, 0, s>>>(a);
         batched_stage_kernel<128, 6, PREC, ROLE_READER><<<ctas, 128, 0, s>>>(a);
         break;
     default:

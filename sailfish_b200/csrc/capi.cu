@@ -87,6 +87,9 @@ Consts cbd::consts_from_grid(const cbd_grid_t *g)
     k.buf_lo2 = k.buf_onset > 0.0 ? k.buf_onset * k.buf_onset * (1.0 - 1e-10) : -1.0;
     k.buf_span = g->buffer_outer_radius - k.buf_onset;
     k.inv_buf_span = 1.0 / k.buf_span;
+    const double key[12] = {20261204.5, 0.0, (double)k.eos, (double)k.ni, (double)k.nj, k.xl,
+                            k.yl,       k.dx, k.dy,          k.cs2,        k.mach2,      k.inv_mach2};
+    std::memcpy(k.cache_key, key, sizeof(key));
     return k;
 }
 

@@ -32,6 +32,7 @@
 
 #include <cuda_runtime.h>
 #include <math.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "../../include/cbdiso_b200.h"
@@ -67,6 +68,7 @@ struct Consts {
     int need_rates;     // epilogue: bit p gravity rates of mass p, bit 2 + p accretion rates
     int rates_only;     // epilogue: every diagnostic is a source rate of the masses, without a radial cut
     cbd_diag_t diag[CBD_MAX_DIAG];
+    double cache_key[12];  // the mesh and EOS part of a face cache's key (slot 1, the precision, by the kernel)
 };
 
 struct MassDev {
@@ -727,54 +729,40 @@ __host__ __device__ inline CacheArrays cache_arrays(double *fc, int ni, int nj)
     return c;
 }
 
-// The key: a format tag, the precision, then every input of the cached values.
-template <int PREC>
-__device__ __forceinline__ double cache_key_value(const Consts &k, const MassDev *m, int v)
-{
-    switch (v) {
-    case 0: return 20261204.5;
-    case 1: return (double)PREC;
-    case 2: return (double)k.eos;
-    case 3: return (double)k.ni;
-    case 4: return (double)k.nj;
-    case 5: return k.xl;
-    case 6: return k.yl;
-    case 7: return k.dx;
-    case 8: return k.dy;
-    case 9: return k.cs2;
-    case 10: return k.mach2;
-    case 11: return k.inv_mach2;
-    default: {
-        const MassDev &q = m[(v - 12) >> 2];
-        switch ((v - 12) & 3) {
-        case 0: return q.x;
-        case 1: return q.y;
-        case 2: return q.mass;
-        default: return q.soft2;
-        }
-    }
-    }
-}
-
 __device__ __forceinline__ bool same_bits(double a, double b)
 {
     return __double_as_longlong(a) == __double_as_longlong(b);
 }
 
+// Word v of the key: a format tag, the precision, then every other input of
+// the cached values (the constants' part is laid out by the host).
 template <int PREC>
-__device__ bool cache_key_matches(const Consts &k, const StageDev &st, const double *fc)
+__device__ __forceinline__ double cache_key_value(const Consts &k, const MassDev *m, int v)
 {
-    for (int v = 0; v < CACHE_KEY; ++v)
-        if (!same_bits(fc[v], cache_key_value<PREC>(k, st.m, v)))
-            return false;
-    return true;
+    if (v < 12)
+        return v == 1 ? (double)PREC : k.cache_key[v];
+    // x, y, mass and soft2 of either mass
+    const int f = (v - 12) & 3;
+    return reinterpret_cast<const double *>(m + ((v - 12) >> 2))[f + (f >> 1) * 2];
+}
+static_assert(offsetof(MassDev, y) == 8 && offsetof(MassDev, mass) == 32 && offsetof(MassDev, soft2) == 40,
+              "cache_key_value indexes MassDev");
+
+// Whether the cache's key is that of the stage's masses: a word per thread,
+// the same answer in all. A barrier of the block.
+template <int PREC>
+__device__ __forceinline__ bool cache_key_matches(const Consts &k, const StageDev &st, const double *fc)
+{
+    const int v = threadIdx.x;
+    return __syncthreads_and(v >= CACHE_KEY || same_bits(fc[v], cache_key_value<PREC>(k, st.m, v)));
 }
 
+// The key written by the first CACHE_KEY threads.
 template <int PREC>
-__device__ void cache_write_key(const Consts &k, const StageDev &st, double *fc)
+__device__ __forceinline__ void cache_write_key(const Consts &k, const StageDev &st, double *fc)
 {
-    for (int v = 0; v < CACHE_KEY; ++v)
-        fc[v] = cache_key_value<PREC>(k, st.m, v);
+    if (threadIdx.x < CACHE_KEY)
+        fc[threadIdx.x] = cache_key_value<PREC>(k, st.m, threadIdx.x);
 }
 
 // The cached values depend on these fields of the masses only (the same
@@ -790,9 +778,9 @@ __device__ __forceinline__ bool same_cached_inputs(const StageDev &st)
 }
 
 // A writer stores the values when its masses are the end-of-step masses (the
-// same answer in every thread); `key_writer` (one thread) then writes the key.
+// same answer in every thread); `key_writer` (one block) then writes the key.
 template <int PREC>
-__device__ bool cache_write_check(const Consts &k, const StageDev &st, double *fc, bool key_writer)
+__device__ __forceinline__ bool cache_write_check(const Consts &k, const StageDev &st, double *fc, bool key_writer)
 {
     const bool end_masses = same_cached_inputs(st);
     if (end_masses && key_writer)
@@ -1233,6 +1221,85 @@ __device__ __forceinline__ void load_record(StageDev &st, const StageDev &param,
         dst[w] = src[w];
 }
 
+// The cached values at mesh point (i, j) for the masses m, with the stage
+// kernel's own expressions: the x-face pair when XF, the y-face pair when YF,
+// the zone's gravity factors when ZONE.
+template <bool FAST>
+__device__ __forceinline__ void face_cache_fill_point(const Consts &k, const MassDev *m, const CacheArrays &c,
+                                                      int i, int j, bool xface, bool yface, bool zone)
+{
+    const int nj = k.nj;
+    const double xf = k.xl + (double)i * k.dx;
+    const double xc = k.xl + ((double)i + 0.5) * k.dx;
+    const double yf = k.yl + (double)j * k.dy;
+    const double yc = k.yl + ((double)j + 0.5) * k.dy;
+    if (xface) {
+        const double cs2 = sound_speed2<FAST>(k, m, xf, yc);
+        cache_store(c.xf + 2 * ((size_t)i * nj + j), cs2, crm::sqrt_rn(cs2));
+    }
+    if (yface) {
+        const double cs2 = sound_speed2<FAST>(k, m, xc, yf);
+        cache_store(c.yf + 2 * ((size_t)i * (nj + 1) + j), cs2, crm::sqrt_rn(cs2));
+    }
+    if (zone) {
+        double g[2] = {0.0, 0.0};
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            if (m[p].mass != 0.0) {
+                const double dx = xc - m[p].x;
+                const double dy = yc - m[p].y;
+                g[p] = inv_pow15<FAST>(dx * dx + dy * dy + m[p].soft2);
+            }
+        }
+        cache_store(c.grav + 2 * ((size_t)i * nj + j), g[0], g[1]);
+    }
+}
+
+// The points of one tile of a grid: columns c0 .. c0 + width - 1 and rows
+// r0 .. r0 + rows - 1, plus column nj in the last strip and row ni in the
+// last segment. All threads of the block take part.
+template <int BJ, bool FAST>
+__device__ __forceinline__ void face_cache_fill_tile(const Consts &k, const MassDev *m, double *fc, int c0,
+                                                     int width, int r0, int rows)
+{
+    const CacheArrays c = cache_arrays(fc, k.ni, k.nj);
+    const int W = min(width, k.nj - c0);
+    const int wext = c0 + W == k.nj ? W + 1 : W;
+    const int r1 = min(r0 + rows, k.ni);
+    const int rext = r1 == k.ni ? r1 + 1 : r1;
+    for (int i = r0; i < rext; ++i)
+        for (int t = threadIdx.x; t < wext; t += BJ)
+            face_cache_fill_point<FAST>(k, m, c, i, c0 + t, t < W, i < r1, i < r1 && t < W);
+}
+
+// Makes the face cache valid for a reader stage: when its key does not match
+// the stage's masses, the CTAs fill the stage's tiles (`strips` x `tiles /
+// strips` of BJ columns x k.rows_per_cta rows), CTA b taking tiles b,
+// b + gridDim.x, ..., with the values for those masses (the reader stage then
+// writes the key). The common case is a matching key: a grid of a few CTAs
+// per SM, the record and the key read a word per thread. (The fill inside the
+// reader, by each tile for itself, saved this launch on small grids, 3 us a
+// step, but its code cost the march 16 bytes of spills, 1.617 -> 1.646 ms
+// per 4096^2 step, and the batched march 130, 835 -> 938 us.) A halted record
+// (a stopped device stepper) fills nothing. The evaluation is long chains of
+// dependent operations: many warps per SM, registers capped to allow them.
+constexpr int FILL_WARPS_PER_SM = 24;
+
+template <int BJ, int PREC>
+__global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ)
+    face_cache_fill_kernel(const Consts k, const StageDev st_param, const StageDev *stage_dev, double *fc, int strips,
+                           int tiles)
+{
+    __shared__ StageDev st;
+    load_record<BJ>(st, st_param, stage_dev);
+    __syncthreads();
+    if (cache_key_matches<PREC>(k, st, fc) || st.halt)
+        return;
+    for (int u = blockIdx.x; u < tiles; u += gridDim.x)
+        face_cache_fill_tile<BJ, PREC == CBD_PRECISION_FAST>(k, st.m, fc, (u % strips) * BJ, BJ,
+                                                             (u / strips) * k.rows_per_cta, k.rows_per_cta);
+}
+
 // One RK stage on one grid: CTA (x, y) marches strip x, segment y. ROLE
 // (ROLE_*) is what the launch does with args.fcache; P2 that k.spacing_pow2
 // is set (the divisions by dx and dy are then the products with their exact
@@ -1248,14 +1315,13 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
     if (st.halt)
         return;
     if (ROLE == ROLE_WRITER) {
-        const bool store = cache_write_check<PREC>(k, st, args.fcache,
-                                                   threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0);
+        const bool store = cache_write_check<PREC>(k, st, args.fcache, blockIdx.x == 0 && blockIdx.y == 0);
         march_tile<BJ, FAST, CACHE_WRITE, true, P2>(k, st, args, c0, BJ, r0, store);
     } else if (ROLE == ROLE_READER) {
         march_tile<BJ, FAST, CACHE_READ, true, P2>(k, st, args, c0, BJ, r0);
         // the fill kernel before this launch made the values valid for these
         // masses; say so for the next fill (no one reads the key meanwhile)
-        if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0)
+        if (blockIdx.x == 0 && blockIdx.y == 0)
             cache_write_key<PREC>(k, st, args.fcache);
     } else {
         march_tile<BJ, FAST, CACHE_NONE, true, P2>(k, st, args, c0, BJ, r0);
@@ -1415,87 +1481,6 @@ __global__ void __launch_bounds__(BJ, epi_warps(RATES) * 32 / BJ)
     double red[PARTIAL_STRIDE];
     block_reduce<BJ, RATES>(acc, sred, red);
     grid_finish<BJ>(red, 1 + 2 * k.num_diag, args.scratch, k.want_ws ? args.result : nullptr, args.result + 1, sred);
-}
-
-// Every cached value at mesh point (i, j), 0 <= i <= ni, 0 <= j <= nj, for
-// the masses m, with the stage kernel's own expressions: the x-face pair
-// (i, j) when j < nj, the y-face pair when i < ni, and the zone's gravity
-// factors when both are inside.
-template <bool FAST>
-__device__ __forceinline__ void face_cache_fill_point(const Consts &k, const MassDev *m, const CacheArrays &c,
-                                                      int i, int j)
-{
-    const int ni = k.ni, nj = k.nj;
-    const double xf = k.xl + (double)i * k.dx;
-    const double xc = k.xl + ((double)i + 0.5) * k.dx;
-    const double yf = k.yl + (double)j * k.dy;
-    const double yc = k.yl + ((double)j + 0.5) * k.dy;
-    if (j < nj) {
-        const double cs2 = sound_speed2<FAST>(k, m, xf, yc);
-        cache_store(c.xf + 2 * ((size_t)i * nj + j), cs2, crm::sqrt_rn(cs2));
-    }
-    if (i < ni) {
-        const double cs2 = sound_speed2<FAST>(k, m, xc, yf);
-        cache_store(c.yf + 2 * ((size_t)i * (nj + 1) + j), cs2, crm::sqrt_rn(cs2));
-    }
-    if (i < ni && j < nj) {
-        double g[2] = {0.0, 0.0};
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            if (m[p].mass != 0.0) {
-                const double dx = xc - m[p].x;
-                const double dy = yc - m[p].y;
-                g[p] = inv_pow15<FAST>(dx * dx + dy * dy + m[p].soft2);
-            }
-        }
-        cache_store(c.grav + 2 * ((size_t)i * nj + j), g[0], g[1]);
-    }
-}
-
-// The points of one tile of a grid: columns c0 .. c0 + width - 1 and rows
-// r0 .. r0 + rows - 1, plus column nj in the last strip and row ni in the
-// last segment. All threads of the block take part.
-template <int BJ, bool FAST>
-__device__ __forceinline__ void face_cache_fill_tile(const Consts &k, const MassDev *m, double *fc, int c0,
-                                                     int width, int r0, int rows)
-{
-    const CacheArrays c = cache_arrays(fc, k.ni, k.nj);
-    const int W = min(width, k.nj - c0);
-    const int wext = c0 + W == k.nj ? W + 1 : W;
-    const int r1 = min(r0 + rows, k.ni);
-    const int rext = r1 == k.ni ? r1 + 1 : r1;
-    for (int i = r0; i < rext; ++i)
-        for (int t = threadIdx.x; t < wext; t += BJ)
-            face_cache_fill_point<FAST>(k, m, c, i, c0 + t);
-}
-
-// Makes the face cache valid for a reader stage: when its key does not match
-// the stage's masses, the CTAs fill the stage's tiles (`strips` x `tiles /
-// strips` of BJ columns x k.rows_per_cta rows), CTA b taking tiles b,
-// b + gridDim.x, ..., with the values for those masses (the reader stage then
-// writes the key). A grid of a few CTAs per SM keeps the common case, a
-// matching key, to one check per CTA. A halted record (a stopped device
-// stepper) fills nothing. The evaluation is long chains of dependent
-// operations: many warps per SM, registers capped to allow them.
-constexpr int FILL_WARPS_PER_SM = 24;
-
-template <int BJ, int PREC>
-__global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ)
-    face_cache_fill_kernel(const Consts k, const StageDev st_param, const StageDev *stage_dev, double *fc, int strips,
-                           int tiles)
-{
-    __shared__ StageDev st;
-    __shared__ int fill;
-    if (threadIdx.x == 0) {
-        st = stage_dev ? *stage_dev : st_param;
-        fill = !st.halt && !cache_key_matches<PREC>(k, st, fc);
-    }
-    __syncthreads();
-    if (!fill)
-        return;
-    for (int u = blockIdx.x; u < tiles; u += gridDim.x)
-        face_cache_fill_tile<BJ, PREC == CBD_PRECISION_FAST>(k, st.m, fc, (u % strips) * BJ, BJ,
-                                                             (u / strips) * k.rows_per_cta, k.rows_per_cta);
 }
 
 }  // namespace cbd

@@ -48,9 +48,9 @@ cudaError_t launch_one_p2(const LaunchShape &s, const Consts &k, const StageDev 
     case ROLE_READER: {
         // the fill over the stage's own tiles, then the stage
         const int tiles = s.grid.x * s.grid.y;
-        const int per_sm = FILL_WARPS_PER_SM * 32 / BJ;
-        const int fill_ctas = tiles < 148 * per_sm ? tiles : 148 * per_sm;
-        face_cache_fill_kernel<BJ, PREC><<<fill_ctas, BJ, 0, stream>>>(k, st, a.stage_dev, a.fcache, s.grid.x, tiles);
+        const int ctas = 148 * (FILL_WARPS_PER_SM * 32 / BJ);
+        face_cache_fill_kernel<BJ, PREC><<<tiles < ctas ? tiles : ctas, BJ, 0, stream>>>(k, st, a.stage_dev, a.fcache,
+                                                                                         s.grid.x, tiles);
         stage_kernel<BJ, MINB, PREC, ROLE_READER, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
         break;
     }
