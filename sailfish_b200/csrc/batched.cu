@@ -27,6 +27,7 @@ __global__ void __launch_bounds__(128) batched_finalize_kernel(const DiskDev *di
                                                                double *results, int result_stride)
 {
     __shared__ double sred[PARTIAL_STRIDE * 4];
+    chain_begin();
     const DiskDev &D = disks[blockIdx.x];
     const int n = D.strips * D.segments;
     double acc[PARTIAL_STRIDE];
@@ -181,9 +182,10 @@ int cbdiso_b200_batched_finalize(const void *disks, int num_disks, const double 
 {
     if (!disks || num_disks <= 0 || !partials || !results || result_stride < 1)
         return CBD_ERR_ARGUMENT;
-    batched_finalize_kernel<<<num_disks, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const DiskDev *>(disks), partials, results, result_stride);
-    return cudaGetLastError() == cudaSuccess ? CBD_OK : CBD_ERR_CUDA;
+    return launch_chained(batched_finalize_kernel, num_disks, 128, 0, static_cast<cudaStream_t>(stream),
+                          static_cast<const DiskDev *>(disks), partials, results, result_stride) == cudaSuccess
+               ? CBD_OK
+               : CBD_ERR_CUDA;
 }
 
 int cbdiso_b200_batched_prologue(void *steppers, int num_disks, const double *results, int result_stride,

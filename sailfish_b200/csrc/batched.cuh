@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs
     __shared__ StageDev st;
     __shared__ int s_unit, s_disk;
     const int t = threadIdx.x;
+    chain_begin();
 
     for (;;) {
         if (t == 0) {
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ) batched_fill_
 {
     __shared__ Consts k;
     __shared__ StageDev st;
+    chain_begin();
     const DiskDev &D = a.disks[blockIdx.x];
     if (D.cache_offset < 0)
         return;
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(BJ, epi_warps(RATES) * 32 / BJ)
     __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
     __shared__ int s_disk;
     const int u = blockIdx.x, t = threadIdx.x;
+    chain_begin();
     if (t == 0)
         s_disk = disk_of_unit(a, u);
     __syncthreads();
@@ -221,24 +224,27 @@ cudaError_t launch_batched_fast(const BatchArgs &a, int ctas, int role, cudaStre
 template <int PREC>
 cudaError_t launch_batched(const BatchArgs &a, int ctas, int role, cudaStream_t s)
 {
+    cudaError_t e = cudaSuccess;
     switch (role) {
     case ROLE_WRITER:
-        batched_stage_kernel<128, 6, PREC, ROLE_WRITER><<<ctas, 128, 0, s>>>(a);
+        e = launch_chained(batched_stage_kernel<128, 6, PREC, ROLE_WRITER>, ctas, 128, 0, s, a);
         break;
     case ROLE_READER:
-        batched_fill_kernel<128, PREC>
-            <<<dim3(a.num_disks, (148 * 6 + a.num_disks - 1) / a.num_disks), 128, 0, s>>>(a);
-        batched_stage_kernel<128, 6, PREC, ROLE_READER><<<ctas, 128, 0, s>>>(a);
+        e = launch_chained(batched_fill_kernel<128, PREC>,
+                           dim3(a.num_disks, (148 * 6 + a.num_disks - 1) / a.num_disks), 128, 0, s, a);
+        if (e == cudaSuccess)
+            e = launch_chained(batched_stage_kernel<128, 6, PREC, ROLE_READER>, ctas, 128, 0, s, a);
         break;
     default:
-        batched_stage_kernel<128, 6, PREC, ROLE_NONE><<<ctas, 128, 0, s>>>(a);
+        e = launch_chained(batched_stage_kernel<128, 6, PREC, ROLE_NONE>, ctas, 128, 0, s, a);
         break;
     }
+    if (e != cudaSuccess || !a.epilogue)
+        return e;
     if (a.epilogue == 2)
-        batched_epilogue_kernel<128, PREC, true><<<a.total_units, 128, 0, s>>>(a, role == ROLE_WRITER);
-    else if (a.epilogue)
-        batched_epilogue_kernel<128, PREC, false><<<a.total_units, 128, 0, s>>>(a, role == ROLE_WRITER);
-    return cudaGetLastError();
+        return launch_chained(batched_epilogue_kernel<128, PREC, true>, a.total_units, 128, 0, s, a,
+                              role == ROLE_WRITER);
+    return launch_chained(batched_epilogue_kernel<128, PREC, false>, a.total_units, 128, 0, s, a, role == ROLE_WRITER);
 }
 
 }  // namespace cbd

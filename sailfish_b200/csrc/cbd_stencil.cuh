@@ -36,6 +36,7 @@
 #include <stdint.h>
 
 #include "../../include/cbdiso_b200.h"
+#include "chain.cuh"
 #include "cr_math.cuh"
 
 namespace cbd {
@@ -1291,6 +1292,7 @@ __global__ void __launch_bounds__(BJ, FILL_WARPS_PER_SM * 32 / BJ)
                            int tiles)
 {
     __shared__ StageDev st;
+    chain_begin();
     load_record<BJ>(st, st_param, stage_dev);
     __syncthreads();
     if (cache_key_matches<PREC>(k, st, fc) || st.halt)
@@ -1309,6 +1311,7 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
 {
     constexpr bool FAST = PREC == CBD_PRECISION_FAST;
     __shared__ StageDev st;
+    chain_begin();
     load_record<BJ>(st, st_param, args.stage_dev);
     const int c0 = blockIdx.x * BJ, r0 = blockIdx.y * k.rows_per_cta;
     __syncthreads();
@@ -1326,6 +1329,7 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
     } else {
         march_tile<BJ, FAST, CACHE_NONE, true, P2>(k, st, args, c0, BJ, r0);
     }
+    chain_end();
 }
 
 // Relative slack of the estimated wavespeeds below. The estimate's sound
@@ -1468,6 +1472,7 @@ __global__ void __launch_bounds__(BJ, epi_warps(RATES) * 32 / BJ)
     constexpr bool FAST = PREC == CBD_PRECISION_FAST;
     __shared__ StageDev st;
     __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
+    chain_begin();
     load_record<BJ>(st, st_param, args.stage_dev);
     __syncthreads();
     if (st.halt)
@@ -1480,6 +1485,7 @@ __global__ void __launch_bounds__(BJ, epi_warps(RATES) * 32 / BJ)
     epilogue_tile<BJ, FAST, RATES>(k, st, args.pwr, grav, blockIdx.x * BJ, BJ, blockIdx.y * k.rows_per_cta, acc);
     double red[PARTIAL_STRIDE];
     block_reduce<BJ, RATES>(acc, sred, red);
+    chain_end();
     grid_finish<BJ>(red, 1 + 2 * k.num_diag, args.scratch, k.want_ws ? args.result : nullptr, args.result + 1, sred);
 }
 

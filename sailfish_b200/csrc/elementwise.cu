@@ -79,6 +79,7 @@ __global__ void __launch_bounds__(BJ) reduce_kernel(const Consts k, const StageD
                                                     double *scratch, double *out0, double *out_rest)
 {
     __shared__ double sred[PARTIAL_STRIDE * (BJ / 32)];
+    chain_begin();
     double acc[PARTIAL_STRIDE];
 #pragma unroll
     for (int v = 0; v < PARTIAL_STRIDE; ++v)
@@ -178,8 +179,7 @@ int reduce_ctas(int ni, int nj)
 cudaError_t launch_reduce(const Consts &k, const StageDev &st, const double *p, double *scratch, double *out0,
                           double *out_rest, cudaStream_t s)
 {
-    reduce_kernel<256><<<reduce_ctas(k.ni, k.nj), 256, 0, s>>>(k, st, p, scratch, out0, out_rest);
-    return cudaGetLastError();
+    return launch_chained(reduce_kernel<256>, reduce_ctas(k.ni, k.nj), 256, 0, s, k, st, p, scratch, out0, out_rest);
 }
 
 }  // namespace cbd

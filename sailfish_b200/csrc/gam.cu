@@ -26,6 +26,7 @@
 #include <cstring>
 
 #include "cbdiso_b200.h"
+#include "chain.cuh"
 #include "cr_math.cuh"
 
 namespace cbd {
@@ -407,14 +408,6 @@ __device__ __forceinline__ double cache_key_value(const Consts &k, const Mass *m
     }
 }
 
-__device__ bool cache_key_matches(const Consts &k, const Mass *m, const double *fc)
-{
-    for (int v = 0; v < CACHE_KEY; ++v)
-        if (__double_as_longlong(fc[v]) != __double_as_longlong(cache_key_value(k, m, v)))
-            return false;
-    return true;
-}
-
 // Phase 1: the per-zone quantities of zone (i0 - 1 + a, j0 - 1 + b) and the
 // face geometry of the tile.
 template <int ROLE>
@@ -615,14 +608,15 @@ __device__ __forceinline__ void stage_phase2(const Consts &k, const Stage &st, c
 // ROLE (ROLE_*) is what the stage does with the face cache `fc`.
 template <int ROLE>
 __global__ void __launch_bounds__(NT, STAGE_MIN_BLOCKS) stage_kernel(Consts k, Stage st,
-                                                                          const double *__restrict__ prd,
+                                                                          const double *prd,
                                                                           const double *pn,
-                                                                          const double *__restrict__ un_all,
+                                                                          const double *un_all,
                                                                           double *pwr, unsigned long long *ws_max,
                                                                           double *fc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StageSmem &sm = *reinterpret_cast<StageSmem *>(smem_raw);
+    cbd::chain_begin();
     const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
     const int ni = k.ni, nj = k.nj;
     const int tid = threadIdx.y * TJ + threadIdx.x;
@@ -679,6 +673,7 @@ __global__ void __launch_bounds__(NT, STAGE_MIN_BLOCKS) stage_kernel(Consts k, S
         if (ws_max)
             ws = max_nan(ws, max_wavespeed(out, div_rn(out[3], out[0]) * k.gamma));
     }
+    cbd::chain_end();
     if (ws_max) {  // uniform over the block
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -701,15 +696,13 @@ __global__ void __launch_bounds__(NT, STAGE_MIN_BLOCKS) stage_kernel(Consts k, S
 // own expressions. CTAs take rows i = blockIdx.x, blockIdx.x + gridDim.x, ...
 __global__ void __launch_bounds__(128) cache_fill_kernel(Consts k, Stage st, double *fc)
 {
-    __shared__ int fill;
-    if (threadIdx.x == 0) {
-        fill = cache_key_matches(k, st.m, fc) ? 0 : 1;
-        if (fill)
-            fc[0] = 0.0;
-    }
-    __syncthreads();
-    if (!fill)
+    cbd::chain_begin();
+    const int v = threadIdx.x;
+    if (__syncthreads_and(v >= CACHE_KEY ||
+                          __double_as_longlong(fc[v]) == __double_as_longlong(cache_key_value(k, st.m, v))))
         return;
+    if (v == 0)
+        fc[0] = 0.0;  // every block compares before its own write, and any order of the others' reads is a mismatch
     const CacheView cv = cache_view(k, fc);
     const int ni = k.ni, nj = k.nj;
     for (int i = blockIdx.x; i <= ni; i += gridDim.x) {
@@ -864,6 +857,7 @@ __device__ __forceinline__ void diag_value(const RedArgs &r, const Diag &d, doub
 __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs r, const double *prim, double *partials)
 {
     __shared__ double sm[RED_VALUES][RED_THREADS];
+    cbd::chain_begin();
     const Consts &k = r.k;
     double v[RED_VALUES];
     for (int q = 0; q < RED_VALUES; ++q)
@@ -896,17 +890,33 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs r, const do
         partials[(size_t)blockIdx.x * RED_VALUES + threadIdx.x] = sm[threadIdx.x][0];
 }
 
-__global__ void finish_kernel(const double *partials, int nblocks, double *result)
+// the blocks' partials to the result: serial in block order, which fixes the sums
+constexpr int FINISH_THREADS = 256, FINISH_CHUNK = 592;
+
+__global__ void __launch_bounds__(FINISH_THREADS) finish_kernel(const double *partials, int nblocks, double *result)
 {
+    // the partials through shared memory (loads of a chunk in flight together),
+    // then one thread per value adds them in block order
+    __shared__ double part[FINISH_CHUNK * RED_VALUES];
+    cbd::chain_begin();
     const int q = threadIdx.x;
-    if (q >= RED_VALUES)
-        return;
     double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) {
-        const double x = partials[(size_t)b * RED_VALUES + q];
-        s = q == 0 ? max_nan(s, x) : s + x;
+    for (int b0 = 0; b0 < nblocks; b0 += FINISH_CHUNK) {
+        const int n = nblocks - b0 < FINISH_CHUNK ? nblocks - b0 : FINISH_CHUNK;
+        for (int w = q; w < n * RED_VALUES; w += FINISH_THREADS)
+            part[w] = partials[(size_t)b0 * RED_VALUES + w];
+        __syncthreads();
+        if (q < RED_VALUES) {
+#pragma unroll 8
+            for (int b = 0; b < n; ++b) {
+                const double x = part[b * RED_VALUES + q];
+                s = q == 0 ? max_nan(s, x) : s + x;
+            }
+        }
+        __syncthreads();
     }
-    result[q] = s;
+    if (q < RED_VALUES)
+        result[q] = s;
 }
 
 // the correctly rounded helpers on device arrays (a test hook)
@@ -1007,12 +1017,13 @@ int launch_role(const Consts &k, const Stage &st, const double *prd, const doubl
     }
     if (ROLE == ROLE_READER) {
         const int rows = k.ni + 1 < 148 * 4 ? k.ni + 1 : 148 * 4;
-        cache_fill_kernel<<<rows, 128, 0, s>>>(k, st, fc);
+        const cudaError_t e = cbd::launch_chained(cache_fill_kernel, rows, 128, 0, s, k, st, fc);
+        if (e != cudaSuccess)
+            return status_of(e);
     }
     const dim3 grid((k.nj + TJ - 1) / TJ, (k.ni + TI - 1) / TI), block(TJ, TI / RPT);
-    stage_kernel<ROLE><<<grid, block, sizeof(StageSmem), s>>>(k, st, prd, pn, un, pwr,
-                                                              reinterpret_cast<unsigned long long *>(ws_max), fc);
-    return status_of(cudaGetLastError());
+    return status_of(cbd::launch_chained(stage_kernel<ROLE>, grid, block, sizeof(StageSmem), s, k, st, prd, pn, un,
+                                         pwr, reinterpret_cast<unsigned long long *>(ws_max), fc));
 }
 
 int launch_stage(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
@@ -1274,9 +1285,10 @@ int cbdgam_b200_reduce(const cbdgam_grid_t *grid, const cbd_mass_t *masses, cons
     }
     r.nd = num_diags;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    reduce_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(r, primitive, scratch);
-    finish_kernel<<<1, 32, 0, s>>>(scratch, RED_BLOCKS, result);
-    return status_of(cudaGetLastError());
+    const cudaError_t e = cbd::launch_chained(reduce_kernel, RED_BLOCKS, RED_THREADS, 0, s, r, primitive, scratch);
+    if (e != cudaSuccess)
+        return status_of(e);
+    return status_of(cbd::launch_chained(finish_kernel, 1, FINISH_THREADS, 0, s, scratch, RED_BLOCKS, result));
 }
 
 }  // extern "C"

@@ -43,31 +43,31 @@ cudaError_t launch_one_p2(const LaunchShape &s, const Consts &k, const StageDev 
         return e;
     switch (role) {
     case ROLE_WRITER:
-        stage_kernel<BJ, MINB, PREC, ROLE_WRITER, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
+        e = launch_chained(stage_kernel<BJ, MINB, PREC, ROLE_WRITER, P2>, s.grid, BJ, smem, stream, k, st, a);
         break;
     case ROLE_READER: {
         // the fill over the stage's own tiles, then the stage
         const int tiles = s.grid.x * s.grid.y;
         const int ctas = 148 * (FILL_WARPS_PER_SM * 32 / BJ);
-        face_cache_fill_kernel<BJ, PREC><<<tiles < ctas ? tiles : ctas, BJ, 0, stream>>>(k, st, a.stage_dev, a.fcache,
-                                                                                         s.grid.x, tiles);
-        stage_kernel<BJ, MINB, PREC, ROLE_READER, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
+        e = launch_chained(face_cache_fill_kernel<BJ, PREC>, tiles < ctas ? tiles : ctas, BJ, 0, stream, k, st,
+                           a.stage_dev, a.fcache, s.grid.x, tiles);
+        if (e != cudaSuccess)
+            return e;
+        e = launch_chained(stage_kernel<BJ, MINB, PREC, ROLE_READER, P2>, s.grid, BJ, smem, stream, k, st, a);
         break;
     }
     default:
-        stage_kernel<BJ, MINB, PREC, ROLE_NONE, P2><<<s.grid, BJ, smem, stream>>>(k, st, a);
+        e = launch_chained(stage_kernel<BJ, MINB, PREC, ROLE_NONE, P2>, s.grid, BJ, smem, stream, k, st, a);
         break;
     }
-    if (k.want_ws || k.num_diag > 0) {
-        // the epilogue over the stage's tiles; a writer's cache holds its masses' factors
-        StageArgs e = a;
-        e.fcache = role == ROLE_WRITER ? a.fcache : nullptr;
-        if (k.rates_only)
-            stage_epilogue_kernel<BJ, PREC, true><<<s.grid, BJ, 0, stream>>>(k, st, e);
-        else
-            stage_epilogue_kernel<BJ, PREC, false><<<s.grid, BJ, 0, stream>>>(k, st, e);
-    }
-    return cudaGetLastError();
+    if (e != cudaSuccess || !(k.want_ws || k.num_diag > 0))
+        return e;
+    // the epilogue over the stage's tiles; a writer's cache holds its masses' factors
+    StageArgs ea = a;
+    ea.fcache = role == ROLE_WRITER ? a.fcache : nullptr;
+    if (k.rates_only)
+        return launch_chained(stage_epilogue_kernel<BJ, PREC, true>, s.grid, BJ, 0, stream, k, st, ea);
+    return launch_chained(stage_epilogue_kernel<BJ, PREC, false>, s.grid, BJ, 0, stream, k, st, ea);
 }
 
 // Grids whose spacings are powers of two take the kernels without the

@@ -2,7 +2,7 @@
 // (sailfish/driver.py:508-510), the RK stage times (cbdiso_2d.py:239) and the
 // binary's Kepler orbit (sailfish/physics/kepler.py:329-366, 414-421) computed
 // on the device, so that a run of steps needs no host round trip and can be
-// captured in a CUDA graph. One single-thread prologue kernel per step writes
+// captured in a CUDA graph. A prologue kernel per step (a warp per grid) writes
 // the stage records that the stage kernels read.
 #include <cmath>
 #include <cstring>
@@ -15,78 +15,98 @@ namespace cbd {
 
 namespace {
 
-// One step's prologue for n independent grids (thread d: grid d). With
-// `finalize`, only records the previous step's time-series row. Otherwise:
-// record the previous row (if any), choose dt, write the stage records of
-// this step, advance the clock.
-__global__ void step_prologue_kernel(StepperDev *steppers, int n, const double *results, int result_stride,
-                                     StageDev *records, double *series, int num_values, int finalize)
+// One step's prologue for n independent grids, a warp each (block d: grid d).
+// With `finalize`, only records the previous step's time-series row.
+// Otherwise: record the previous row (if any), choose dt, write the stage
+// records of this step, advance the clock. Lane k solves the orbit at stage
+// k's time and lane num_stages at the end of the step: the four solves, each a
+// serial chain of sines and cosines, run side by side (one thread took 10 us a
+// step), and the records leave a word per lane.
+__global__ void __launch_bounds__(32) step_prologue_kernel(StepperDev *steppers, const double *results,
+                                                           int result_stride, StageDev *records, double *series,
+                                                           int num_values, int finalize)
 {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= n)
-        return;
+    __shared__ MassDev mass[4][2];
+    __shared__ StageDev out[3];
+    chain_begin();
+    const int d = blockIdx.x, lane = threadIdx.x;
     StepperDev *s = steppers + d;
     const double *result = results + (size_t)d * result_stride;
+    const int step = s->step;
     if (s->status != CBD_OK)
         return;
-    if (s->step > 0 && series && s->step - 1 < s->series_capacity) {
-        double *row = series + ((size_t)d * s->series_capacity + (s->step - 1)) * (3 + num_values);
-        row[0] = s->time;
-        row[1] = s->dt;
-        row[2] = result[0];
-        for (int v = 0; v < num_values; ++v)
-            row[3 + v] = result[1 + v];
+    if (step > 0 && series && step - 1 < s->series_capacity) {
+        double *row = series + ((size_t)d * s->series_capacity + (step - 1)) * (3 + num_values);
+        for (int v = lane; v < 3 + num_values; v += 32)
+            row[v] = v == 0 ? s->time : v == 1 ? s->dt : result[v - 2];
     }
     if (finalize)
         return;
-    if (s->dt_sequence && s->step >= s->dt_count) {
-        s->status = CBD_ERR_ARGUMENT;
+    __syncwarp();  // every lane has read the fields that lane 0 may write
+    if (s->dt_sequence && step >= s->dt_count) {
+        if (lane == 0)
+            s->status = CBD_ERR_ARGUMENT;
         return;
     }
-    const double dt = s->dt_sequence ? s->dt_sequence[s->step]
+    const double dt = s->dt_sequence ? s->dt_sequence[step]
                                      : (s->fixed_dt > 0.0 ? s->fixed_dt : s->min_spacing / result[0] * s->cfl);
-    StageDev *rec = records + (size_t)d * s->num_stages;
+    const int num_stages = s->num_stages;
+    StageDev *rec = records + (size_t)d * num_stages;
     if (!(isfinite(dt) && dt > 0.0)) {
         // a NaN, infinite or zero wavespeed (or a bad dt sequence entry):
         // stop here, and make the stages of this and every later step of a
         // captured sequence leave the state as it is
-        s->status = CBD_ERR_NONFINITE;
-        for (int k = 0; k < s->num_stages; ++k)
-            rec[k].halt = 1;
+        if (lane < num_stages)
+            rec[lane].halt = 1;
+        if (lane == 0)
+            s->status = CBD_ERR_NONFINITE;
         return;
     }
     const double time0 = s->time;
-    double t = time0;
-    double times[3];
-    for (int k = 0; k < s->num_stages; ++k) {
-        times[k] = t;
+    double t = time0, mine = time0;
+    for (int k = 0; k < num_stages; ++k) {
         t = time0 * s->weights[k] + (t + dt) * (1.0 - s->weights[k]);
+        if (lane == k + 1)
+            mine = t;
     }
-    MassDev end[2];
-    if (!orbit_masses(s->orbit, t, end)) {
-        s->status = CBD_ERR_KEPLER;
+    const bool solved = lane > num_stages || orbit_masses(s->orbit, mine, mass[lane]);
+    if (!__all_sync(0xffffffffu, solved)) {
+        if (lane == 0)
+            s->status = CBD_ERR_KEPLER;
         return;
     }
-    for (int k = 0; k < s->num_stages; ++k) {
-        StageDev &r = rec[k];
-        if (!orbit_masses(s->orbit, times[k], r.m)) {
-            s->status = CBD_ERR_KEPLER;
-            return;
-        }
-        r.e[0] = end[0];
-        r.e[1] = end[1];
-        r.a = s->weights[k];
-        r.one_minus_a = 1.0 - s->weights[k];
+    if (lane < num_stages) {
+        StageDev &r = out[lane];
+        r.m[0] = mass[lane][0];
+        r.m[1] = mass[lane][1];
+        r.e[0] = mass[num_stages][0];
+        r.e[1] = mass[num_stages][1];
+        r.a = s->weights[lane];
+        r.one_minus_a = 1.0 - s->weights[lane];
         r.dt = dt;
         r.buffer_mass = r.m[0].mass + r.m[1].mass;
         r.buffer_k = s->buffer_k;
         r.halt = 0;
-        if (s->history && s->step < s->history_capacity)
-            s->history[(size_t)s->step * s->num_stages + k] = r;
+        r._pad = 0;
     }
-    s->dt = dt;
-    s->time = t;
-    s->step += 1;
+    __syncwarp();
+    const int words = num_stages * (int)(sizeof(StageDev) / sizeof(double));
+    const double *src = reinterpret_cast<const double *>(out);
+    double *dst = reinterpret_cast<double *>(rec);
+    double *hist = s->history && step < s->history_capacity
+                       ? reinterpret_cast<double *>(s->history + (size_t)step * num_stages)
+                       : nullptr;
+    for (int w = lane; w < words; w += 32) {
+        dst[w] = src[w];
+        if (hist)
+            hist[w] = src[w];
+    }
+    __syncwarp();
+    if (lane == 0) {
+        s->dt = dt;
+        s->time = t;
+        s->step = step + 1;
+    }
 }
 
 }  // namespace
@@ -95,9 +115,8 @@ cudaError_t launch_step_prologue(StepperDev *s, int n, const double *results, in
                                  StageDev *records, double *series, int num_values, int finalize,
                                  cudaStream_t stream)
 {
-    step_prologue_kernel<<<(n + 63) / 64, 64, 0, stream>>>(s, n, results, result_stride, records, series,
-                                                           num_values, finalize);
-    return cudaGetLastError();
+    return launch_chained(step_prologue_kernel, n, 32, 0, stream, s, results, result_stride, records, series,
+                          num_values, finalize);
 }
 
 }  // namespace cbd
