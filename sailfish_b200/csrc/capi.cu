@@ -102,6 +102,33 @@ double buffer_k(double driving_rate, double central_mass, double onset)
     return driving_rate * std::sqrt(central_mass * std::pow(onset, -3.0));
 }
 
+// Rows per CTA on a grid small enough for one wave of short segments: there a
+// launch takes as long as one CTA's march, r rows and the lead-in of about one
+// row's work, at a time per row that grows with the 128-thread CTAs c that the
+// fullest SM holds. (r + 1.1) (3 + 1.25 c) ranks the measured steps (us, rows 1 / 2 / 3 /
+// 4 / 6 / 8): 64^2 26 / 31 / 37 / 43 / 54 / 65, 128^2 27 / 32 / 38 / 43 / 53 /
+// 64, 256^2 33 / 35 / 41 / 44 / 55 / 65, 384^2 55 / 43 / 46 / 49 / 62 / 69
+// (one row: two waves), 512^2 79 / 68 / 59 / 60 / 68 / 74, 640^2 111 / 86 /
+// 85 / 80 / 80 / 86, 768^2 150 / 116 / 107 / 107 / 106 / 99. 0: not such a
+// grid (one wave takes more than 8 rows; from 1024^2 the rule below).
+int small_grid_rows(int ni, int strips, int bj, int slots)
+{
+    int best = 0;
+    double least = 0.0;
+    for (int r = 1; r <= 8; ++r) {
+        const long ctas = (long)strips * ((ni + r - 1) / r);
+        if (ctas > slots)
+            continue;
+        const double c = (double)((ctas + 147) / 148) * bj / 128.0;
+        const double cost = (r + 1.1) * (3.0 + 1.25 * c);
+        if (best == 0 || cost < least) {
+            best = r;
+            least = cost;
+        }
+    }
+    return best;
+}
+
 // Launch shape of the stage kernel. Defaults: 256-column strips (3 resident
 // CTAs per SM) on grids of at least 2048^2 zones, 128-column strips compiled
 // for 6 resident CTAs per SM below that (64-column strips and 12 CTAs for
@@ -110,6 +137,7 @@ double buffer_k(double driving_rate, double central_mass, double onset)
 // 0.637 ms with 256 columns; 1024^2 0.232 -> 0.234 ms.)
 LaunchShape stage_shape(int ni, int nj, int bj, int rows, int occupancy = 0)
 {
+    const bool chosen = rows <= 0;
     LaunchShape s;
     if (bj != 64 && bj != 128 && bj != 256) {
         bj = nj >= 2048 && (long)ni * nj >= 2048L * 2048 ? 256 : (nj > 96 ? 128 : 64);
@@ -137,6 +165,10 @@ LaunchShape stage_shape(int ni, int nj, int bj, int rows, int occupancy = 0)
         // 5 rows in 1.85 waves 0.219 ms). Score of r rows in W waves:
         // (W / ceil(W)) (r / (r + 2)), times 0.95 below 1.5 waves.
         const int slots = 148 * (s.minb > 1 ? s.minb : 4);
+        rows = small_grid_rows(ni, strips, bj, slots);
+    }
+    if (rows <= 0) {
+        const int slots = 148 * (s.minb > 1 ? s.minb : 4);
         rows = 4;
         double best = -1.0;
         for (int r = 48; r >= 4; --r) {
@@ -148,7 +180,7 @@ LaunchShape stage_shape(int ni, int nj, int bj, int rows, int occupancy = 0)
             }
         }
     }
-    if (rows < 4)
+    if (rows < 4 && !chosen)
         rows = 4;
     s.bj = bj;
     s.rows = rows;
@@ -404,8 +436,12 @@ size_t cbdiso_b200_scratch_bytes(const cbd_grid_t *grid)
 {
     if (!valid_grid(grid))
         return 0;
+    // the finest explicit shape; the shorter segments of small_grid_rows stay
+    // within one wave, at most 148 * 12 CTAs
     const LaunchShape s = stage_shape(grid->ni, grid->nj, 64, 4);
     size_t ctas = (size_t)s.grid.x * s.grid.y;
+    if (ctas < 148 * 12)
+        ctas = 148 * 12;
     const size_t r = (size_t)reduce_ctas(grid->ni, grid->nj);
     if (r > ctas)
         ctas = r;
