@@ -129,6 +129,41 @@ int small_grid_rows(int ni, int strips, int bj, int slots)
     return best;
 }
 
+}  // namespace
+
+// Rows per CTA of a marching stage kernel on a grid of ni rows and `strips`
+// strips, `slots` CTAs of bj threads resident at a time.
+//
+// Beyond the small grids the CTAs should fill whole waves of the resident
+// slots: a last, partial wave leaves SMs idle at the end of the launch (4096^2
+// at 256 columns: 37 rows, 4.0 waves, 2.127 ms per step; 36 rows, 4.11
+// waves, 2.239 ms; 32 rows, 4.61 waves, 2.150 ms). Each CTA also
+// recomputes about two rows' worth of slopes and faces at its
+// segment's top, and a single wave starts every CTA at once
+// (2048^2: 19 rows in 1.95 waves 0.607 ms, 38 rows in 0.97 waves
+// 0.628 ms; 1024^2 at 128 columns: 10 rows in 0.93 waves 0.212 ms,
+// 5 rows in 1.85 waves 0.219 ms). Score of r rows in W waves:
+// (W / ceil(W)) (r / (r + 2)), times 0.95 below 1.5 waves.
+int cbd::segment_rows(int ni, int strips, int bj, int slots)
+{
+    const int small = small_grid_rows(ni, strips, bj, slots);
+    if (small > 0)
+        return small;
+    int rows = 4;
+    double best = -1.0;
+    for (int r = 48; r >= 4; --r) {
+        const double waves = (double)strips * ((ni + r - 1) / r) / slots;
+        const double score = waves / std::ceil(waves) * r / (r + 2.0) * (waves < 1.5 ? 0.95 : 1.0);
+        if (score > best * (1.0 + 1e-3)) {
+            best = score;
+            rows = r;
+        }
+    }
+    return rows;
+}
+
+namespace {
+
 // Launch shape of the stage kernel. Defaults: 256-column strips (3 resident
 // CTAs per SM) on grids of at least 2048^2 zones, 128-column strips compiled
 // for 6 resident CTAs per SM below that (64-column strips and 12 CTAs for
@@ -153,33 +188,8 @@ LaunchShape stage_shape(int ni, int nj, int bj, int rows, int occupancy = 0)
     if (bj == 64 && (occupancy == 10 || occupancy == 12))
         s.minb = occupancy;
     const int strips = (nj + bj - 1) / bj;
-    if (rows <= 0) {
-        // The CTAs should fill whole waves of the resident slots: a last,
-        // partial wave leaves SMs idle at the end of the launch (4096^2 at
-        // 256 columns: 37 rows, 4.0 waves, 2.127 ms per step; 36 rows, 4.11
-        // waves, 2.239 ms; 32 rows, 4.61 waves, 2.150 ms). Each CTA also
-        // recomputes about two rows' worth of slopes and faces at its
-        // segment's top, and a single wave starts every CTA at once
-        // (2048^2: 19 rows in 1.95 waves 0.607 ms, 38 rows in 0.97 waves
-        // 0.628 ms; 1024^2 at 128 columns: 10 rows in 0.93 waves 0.212 ms,
-        // 5 rows in 1.85 waves 0.219 ms). Score of r rows in W waves:
-        // (W / ceil(W)) (r / (r + 2)), times 0.95 below 1.5 waves.
-        const int slots = 148 * (s.minb > 1 ? s.minb : 4);
-        rows = small_grid_rows(ni, strips, bj, slots);
-    }
-    if (rows <= 0) {
-        const int slots = 148 * (s.minb > 1 ? s.minb : 4);
-        rows = 4;
-        double best = -1.0;
-        for (int r = 48; r >= 4; --r) {
-            const double waves = (double)strips * ((ni + r - 1) / r) / slots;
-            const double score = waves / std::ceil(waves) * r / (r + 2.0) * (waves < 1.5 ? 0.95 : 1.0);
-            if (score > best * (1.0 + 1e-3)) {
-                best = score;
-                rows = r;
-            }
-        }
-    }
+    if (rows <= 0)
+        rows = cbd::segment_rows(ni, strips, bj, 148 * (s.minb > 1 ? s.minb : 4));
     if (rows < 4 && !chosen)
         rows = 4;
     s.bj = bj;

@@ -26,6 +26,9 @@ cudaError_t launch_stage_fast(const LaunchShape &s, const Consts &k, const Stage
 Consts consts_from_grid(const cbd_grid_t *g);
 int set_diagnostics(Consts &k, const cbd_epilogue_t *ep, int first, int count);
 
+// Rows per CTA of a marching stage kernel (capi.cu).
+int segment_rows(int ni, int strips, int bj, int slots);
+
 // The stream the drop-in kernels launch on (cbdiso_b200_set_stream).
 cudaStream_t drop_in_stream();
 

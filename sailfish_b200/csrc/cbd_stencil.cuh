@@ -36,6 +36,7 @@
 #include <stdint.h>
 
 #include "../../include/cbdiso_b200.h"
+#include "async.cuh"
 #include "chain.cuh"
 #include "cr_math.cuh"
 
@@ -629,34 +630,6 @@ __device__ void grid_finish(const double (&mine)[PARTIAL_STRIDE], int n, double 
 }
 
 // ---------------------------------------------------------------------------
-// asynchronous global -> shared copies (cp.async), used to fetch the next row
-// of the march one iteration ahead of its use
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ void async_copy8(void *smem, const void *gmem)
-{
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
-__device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-
-__device__ __forceinline__ void async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-__device__ __forceinline__ void async_copy16(void *smem, const void *gmem)
-{
-    const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-
-// waits until at most N of this thread's most recent groups are in flight
-template <int N>
-__device__ __forceinline__ void async_wait()
-{
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
-// ---------------------------------------------------------------------------
 // the fused stage kernel
 // ---------------------------------------------------------------------------
 
@@ -934,7 +907,7 @@ __device__ __forceinline__ void march_tile(const Consts &k, const StageDev &st, 
         fetch_row(1, r0 - 1);
         fetch_row(2, r0);
         async_commit();
-        async_wait_all();
+        async_wait<0>();
         __syncthreads();
         if (r0 + 1 <= r1 + 1)
             fetch_row(3, r0 + 1);
@@ -950,7 +923,7 @@ __device__ __forceinline__ void march_tile(const Consts &k, const StageDev &st, 
 
     for (int r = r0 - 2; r < r1; ++r) {
         if constexpr (!ONE_SYNC) {
-            async_wait_all();
+            async_wait<0>();
             __syncthreads();
             if (r + 3 <= r1 + 1)
                 fetch_row((r + 3) & 3, r + 3);
@@ -1095,7 +1068,7 @@ __device__ __forceinline__ void march_tile(const Consts &k, const StageDev &st, 
         if constexpr (ONE_SYNC) {
             // row r + 3 has landed for this thread; after the barrier for
             // all, and the slot of row r - 1 is free for row r + 4
-            async_wait_all();
+            async_wait<0>();
             __syncthreads();
             if (r + 4 <= r1 + 1) {
                 const int s4 = s2 >= 3 ? s2 - 3 : s2 + 2;  // (s0 + 4) mod 5
