@@ -28,6 +28,8 @@
 namespace cbd {
 
 constexpr int NPAR = 12;  // m1 (x, y, vx, vy, mass), m2 (...), nu, sink rate
+constexpr int ADJ_THREADS = 128;
+constexpr int ADJ_MIN_BLOCKS = 5;  // resident blocks per SM the register budget allows
 
 namespace {
 
@@ -244,8 +246,8 @@ struct ParAcc<true> {
     __device__ __forceinline__ void add(int r, double x)
     {
         if (r < 10) {
-            v[0] += x * jac[2 * r];
-            v[1] += x * jac[2 * r + 1];
+            v[0] = fma(x, jac[2 * r], v[0]);
+            v[1] = fma(x, jac[2 * r + 1], v[1]);
         } else {
             v[r - 8] += x;
         }
@@ -270,7 +272,7 @@ template <class Acc>
 __device__ __forceinline__ void cs2_param_vjp(const Consts &k, const StageDev &st, double x, double y, double lam,
                                               Acc &par)
 {
-    if (k.eos != 2 || lam == 0.0)
+    if (k.eos != 2)
         return;
     const double l = lam * k.inv_mach2;
     for (int p = 0; p < 2; ++p) {
@@ -278,7 +280,7 @@ __device__ __forceinline__ void cs2_param_vjp(const Consts &k, const StageDev &s
         if (!(m.mass > 0.0))
             continue;
         const double dx = x - m.x, dy = y - m.y;
-        const double s12 = rsqrt(dx * dx + dy * dy + m.soft2);
+        const double s12 = crm::rsqrt_near(dx * dx + dy * dy + m.soft2);
         const double w = l * m.mass * s12 * s12 * s12;
         par.add(5 * p + 0, w * dx);
         par.add(5 * p + 1, w * dy);
@@ -302,7 +304,7 @@ __device__ __forceinline__ void hlle_vjp(const double *pl, const double *pr, dou
     const unsigned s_am = sel & 3u, s_ap = (sel >> 2) & 3u;
     const double am = s_am == 0 ? 0.0 : (s_am == 1 ? vl - cs : vr - cs);
     const double ap = s_ap == 0 ? 0.0 : (s_ap == 1 ? vl + cs : vr + cs);
-    const double inv_d = 1.0 / (ap - am);
+    const double inv_d = crm::recip_rn(ap - am);
     double lfl[3], lfr[3], lul[3], lur[3], lap = 0.0, lam = 0.0;
     for (int q = 0; q < 3; ++q) {
         const double F = (fl[q] * ap - fr[q] * am - (ul[q] - ur[q]) * ap * am) * inv_d;
@@ -330,7 +332,7 @@ __device__ __forceinline__ void hlle_vjp(const double *pl, const double *pr, dou
         lcs += lap;
     }
     if (cs > 0.0)
-        *lcs2 += lcs * (0.5 / cs);
+        *lcs2 += lcs * (0.5 * crm::recip_rn(cs));
     // fluxes: f0 = v u0, f1 = v u1 (+ rho cs2 if DIR == 0), f2 = v u2 (+ rho cs2 if DIR == 1)
     lvl += lfl[0] * ul[0] + lfl[1] * ul[1] + lfl[2] * ul[2];
     lvr += lfr[0] * ur[0] + lfr[1] * ur[1] + lfr[2] * ur[2];
@@ -368,7 +370,7 @@ __device__ __forceinline__ void gravity_vjp(const MassDev &m, int p, double x, d
     if (m.mass == 0.0)
         return;
     const double dx = x - m.x, dy = y - m.y;
-    const double r = rsqrt(dx * dx + dy * dy + m.soft2);
+    const double r = crm::rsqrt_near(dx * dx + dy * dy + m.soft2);
     const double g = r * r * r;
     const double h = g * r * r;
     const double sig = pc[0];
@@ -406,7 +408,7 @@ __device__ __forceinline__ void lam_rk_zone(const Consts &k, const double *o, co
 {
     const bool floor = !(o[0] > k.rho_min);
     const bool ceil_x = !(fabs(o[1]) < k.vmax), ceil_y = !(fabs(o[2]) < k.vmax);
-    const double inv_rho = 1.0 / o[0];
+    const double inv_rho = crm::recip_rn(o[0]);
     const double lvx = ceil_x ? 0.0 : l[1];
     const double lvy = ceil_y ? 0.0 : l[2];
     lu[1] = lvx * inv_rho;
@@ -436,10 +438,10 @@ struct StageShared {
 template <bool CHAIN>
 __device__ __forceinline__ void load_stage(const AdjArgs &a, StageShared &sh)
 {
-    if (threadIdx.x == 0)
-        sh.st = *a.st;
-    if (CHAIN && threadIdx.x >= 32 && threadIdx.x < 52)
-        sh.jac[threadIdx.x - 32] = a.jac[threadIdx.x - 32];
+    chain_begin();
+    load_record<ADJ_THREADS>(sh.st, sh.st, a.st);
+    if (CHAIN && threadIdx.x >= 64 && threadIdx.x < 84)
+        sh.jac[threadIdx.x - 64] = a.jac[threadIdx.x - 64];
     __syncthreads();
 }
 
@@ -477,9 +479,6 @@ __device__ __forceinline__ void store_params(const AdjArgs &a, const ParAcc<CHAI
 __device__ __forceinline__ long grid_start(int nt) { return blockIdx.x * (long)nt + threadIdx.x; }
 __device__ __forceinline__ long grid_step(int nt) { return (long)gridDim.x * nt; }
 
-constexpr int ADJ_THREADS = 128;
-constexpr int ADJ_MIN_BLOCKS = 5;  // resident blocks per SM the register budget allows
-
 // rho * strain (xx, xy, yy) of a zone from its slopes gx, gy (shear_strain,
 // cbdiso_2d.c:248-263, with the constant divisors as reciprocals: derivative
 // arithmetic needs no correct rounding)
@@ -513,7 +512,7 @@ __device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, co
         pr[q] = pR[q] - 0.5 * gR[q];
         lf[q] = (lur[q] - lul[q]) * cf;
     }
-    const double cs2 = cs2_generic(k, m, xf, yf), cs = sqrt(cs2);
+    const double cs2 = cs2_generic(k, m, xf, yf), cs = crm::sqrt_rn(cs2);
     double lpl[3] = {0, 0, 0}, lpr[3] = {0, 0, 0}, lcs2 = 0.0;
     hlle_vjp<DIR>(pl, pr, cs2, cs, hlle_select(pl[1 + DIR], pr[1 + DIR], cs), lf, lpl, lpr, &lcs2);
     cs2_param_vjp(k, st, xf, yf, lcs2, par);
@@ -1025,10 +1024,9 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
                     const double *pp = sm.p[mod(R + 1, 4)][t + 1];
                     const double *pw = sm.p[mod(R, 4)][t], *pe = sm.p[mod(R, 4)][t + 2];
                     for (int q = 0; q < 3; ++q) {
-                        const unsigned sx = slope_select(pm[q], p0[q], pp[q], k.theta);
-                        const unsigned sy = slope_select(pw[q], p0[q], pe[q], k.theta);
-                        o[q] = slope_generic(pm[q], p0[q], pp[q], k.theta);
-                        o[3 + q] = slope_generic(pw[q], p0[q], pe[q], k.theta);
+                        unsigned sx, sy;
+                        o[q] = slope_selected(pm[q], p0[q], pp[q], k.theta, sx);
+                        o[3 + q] = slope_selected(pw[q], p0[q], pe[q], k.theta, sy);
                         w |= sx << (2 * q);
                         w |= sy << (6 + 2 * q);
                     }
@@ -1128,6 +1126,7 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
         }
         __syncthreads();
     }
+    chain_end();
     store_params<AM_NT, CHAIN>(a, par, blockIdx.y * gridDim.x + blockIdx.x);
 }
 
@@ -1240,7 +1239,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) objective_adjoint
             // T = -sigma m g (x dy - y dx)
             if (b.mass != 0.0) {
                 const double dx = x - b.x, dy = y - b.y;
-                const double r = rsqrt(dx * dx + dy * dy + b.soft2);
+                const double r = crm::rsqrt_near(dx * dx + dy * dy + b.soft2);
                 const double g = r * r * r, h = g * r * r;
                 const double cr = x * dy - y * dx;
                 lam[c] += w * (-b.mass * g * cr);
@@ -1437,8 +1436,11 @@ int stage_adjoint_impl(const cbd_grid_t *grid, const void *stage_dev, const doub
         if (jac) {
             if (!march_ready<true>())
                 return CBD_ERR_CUDA;
-            adj_march<true><<<grid, AM_NT, smem, s>>>(k, a, seg);
-            adj_sinks<true><<<bs, T, 0, s>>>(k, a);
+            cudaError_t e = launch_chained(adj_march<true>, grid, AM_NT, smem, s, k, a, seg);
+            if (e == cudaSuccess)
+                e = launch_chained(adj_sinks<true>, bs, T, 0, s, k, a);
+            if (e != cudaSuccess)
+                return CBD_ERR_CUDA;
         } else {
             if (!march_ready<false>())
                 return CBD_ERR_CUDA;
@@ -1485,8 +1487,11 @@ int objective_adjoint_impl(const cbd_grid_t *grid, const void *stage_dev, const 
     constexpr int T = ADJ_THREADS;
     if (jac) {
         a.par = params_out;
-        objective_adjoint_kernel<true><<<bz, T, 0, s>>>(k, a, w_torque, true);
-        objective_sinks<true><<<bs, T, 0, s>>>(k, a, w_mdot, true);
+        cudaError_t e = launch_chained(objective_adjoint_kernel<true>, bz, T, 0, s, k, a, w_torque, true);
+        if (e == cudaSuccess)
+            e = launch_chained(objective_sinks<true>, bs, T, 0, s, k, a, w_mdot, true);
+        if (e != cudaSuccess)
+            return CBD_ERR_CUDA;
     } else {
         objective_adjoint_kernel<false><<<bz, T, 0, s>>>(k, a, w_torque, false);
         sum_params<<<1, 32 * NPAR, 0, s>>>(parts, bz, NPAR, params_out);

@@ -32,7 +32,7 @@ __device__ __forceinline__ Dual operator*(Dual a, Dual b) { return {a.v * b.v, a
 __device__ __forceinline__ Dual operator/(Dual a, Dual b)
 {
     const double q = div_rn<false>(a.v, b.v);
-    return {q, (a.d - q * b.d) / b.v};
+    return {q, div_rn<false>(a.d - q * b.d, b.v)};
 }
 __device__ __forceinline__ Dual operator+(Dual a, double b) { return {a.v + b, a.d}; }
 __device__ __forceinline__ Dual operator+(double a, Dual b) { return {a + b.v, b.d}; }
@@ -40,22 +40,24 @@ __device__ __forceinline__ Dual operator-(Dual a, double b) { return {a.v - b, a
 __device__ __forceinline__ Dual operator-(double a, Dual b) { return {a - b.v, -b.d}; }
 __device__ __forceinline__ Dual operator*(Dual a, double b) { return {a.v * b, a.d * b}; }
 __device__ __forceinline__ Dual operator*(double a, Dual b) { return {a * b.v, a * b.d}; }
-__device__ __forceinline__ Dual operator/(Dual a, double b) { return {div_rn<false>(a.v, b), a.d / b}; }
+__device__ __forceinline__ Dual operator/(Dual a, double b) { return {div_rn<false>(a.v, b), div_rn<false>(a.d, b)}; }
 __device__ __forceinline__ Dual operator/(double a, Dual b)
 {
     const double q = div_rn<false>(a, b.v);
-    return {q, -q * b.d / b.v};
+    return {q, div_rn<false>(-q * b.d, b.v)};
 }
 
 // scalar functions on both types
 __device__ __forceinline__ double g_div(double a, double b) { return div_rn<false>(a, b); }
 __device__ __forceinline__ Dual g_div(Dual a, Dual b) { return a / b; }
-__device__ __forceinline__ double g_sqrt(double x) { return sqrt(x); }
+__device__ __forceinline__ double g_sqrt(double x) { return crm::sqrt_rn(x); }
 __device__ __forceinline__ Dual g_sqrt(Dual x)
 {
-    const double s = sqrt(x.v);
-    return {s, x.d / (2.0 * s)};
+    const double s = crm::sqrt_rn(x.v);
+    return {s, div_rn<false>(x.d, 2.0 * s)};
 }
+__device__ __forceinline__ double g_over_sqrt(double m, double s) { return crm::over_sqrt_rn(m, s); }
+__device__ __forceinline__ Dual g_over_sqrt(Dual m, Dual s) { return m / g_sqrt(s); }
 __device__ __forceinline__ double g_exp(double x) { return exp(x); }
 __device__ __forceinline__ Dual g_exp(Dual x)
 {
@@ -66,7 +68,7 @@ __device__ __forceinline__ double g_pow15(double x) { return inv_pow15<false>(x)
 __device__ __forceinline__ Dual g_pow15(Dual x)
 {
     const double p = inv_pow15<false>(x.v);
-    return {p, -1.5 * p / x.v * x.d};
+    return {p, div_rn<false>(-1.5 * p, x.v) * x.d};
 }
 __device__ __forceinline__ double g_pow4(double q) { return pow4_rn(q); }
 __device__ __forceinline__ Dual g_pow4(Dual q) { return {pow4_rn(q.v), 4.0 * q.v * q.v * q.v * q.d}; }
@@ -112,6 +114,23 @@ __device__ __forceinline__ unsigned slope_select(double yl, double y0, double yr
     return fa < mi ? 1u : inner;
 }
 
+// The limited slope and its selection together (value 0 for selection 0).
+__device__ __forceinline__ double slope_selected(double yl, double y0, double yr, double theta, unsigned &sel)
+{
+    const double a = (y0 - yl) * theta;
+    const double b = (yr - yl) * 0.5;
+    const double c = (yr - y0) * theta;
+    const int ha = __double2hiint(a), hb = __double2hiint(b), hc = __double2hiint(c);
+    const bool same = ((ha ^ hb) | (ha ^ hc)) >= 0;
+    const double fa = fabs(a), fb = fabs(b), fc = fabs(c);
+    const bool b_less = fb < fc;
+    const double mi = b_less ? fb : fc;
+    const bool first = fa < mi;
+    sel = same ? (first ? 1u : (b_less ? 2u : 3u)) : 0u;
+    const double v = first ? a : (b_less ? b : c);
+    return same ? v : 0.0;
+}
+
 template <class T>
 __device__ __forceinline__ T slope_generic(const T &yl, const T &y0, const T &yr, double theta)
 {
@@ -147,7 +166,7 @@ __device__ __forceinline__ T potential_generic(const MassT<T> *m, const T &x, co
             const T dx = x - m[p].x;
             const T dy = y - m[p].y;
             const T r2 = dx * dx + dy * dy;
-            phi = phi - g_div(m[p].mass, g_sqrt(r2 + m[p].base->soft2));
+            phi = phi - g_over_sqrt(m[p].mass, r2 + m[p].base->soft2);
         }
     }
     return phi;

@@ -70,10 +70,10 @@ __device__ __forceinline__ void buffer_generic(const Consts &k, const StageDev &
     const double r2 = x * x + y * y;
     if (!(r2 > k.buf_lo2))
         return;
-    const double rc = sqrt(r2);
+    const double rc = crm::sqrt_rn(r2);
     if (!(rc > k.buf_onset))
         return;
-    const double vk = sqrt(div_rn<false>(st.buffer_mass, rc));
+    const double vk = crm::sqrt_rn(div_rn<false>(st.buffer_mass, rc));
     const double t[3] = {k.buf_sigma, k.buf_sigma * div_rn<false>(-y, rc) * vk,
                          k.buf_sigma * div_rn<false>(+x, rc) * vk};
     const double rate = div_by<false>(st.buffer_k * (rc - k.buf_onset), k.buf_span, k.inv_buf_span);
@@ -89,7 +89,7 @@ __device__ __forceinline__ double buffer_rate(const Consts &k, const StageDev &s
     const double r2 = x * x + y * y;
     if (!(r2 > k.buf_lo2))
         return 0.0;
-    const double rc = sqrt(r2);
+    const double rc = crm::sqrt_rn(r2);
     if (!(rc > k.buf_onset))
         return 0.0;
     return div_by<false>(st.buffer_k * (rc - k.buf_onset), k.buf_span, k.inv_buf_span);
