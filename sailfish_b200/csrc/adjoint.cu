@@ -254,16 +254,17 @@ struct ParAcc<true> {
     }
 };
 
-// An accumulator that counts only when `on` (halo work recomputed by a
-// neighbouring CTA must not be counted twice).
+// Collects one face's or zone's contributions and counts them only when `on`
+// (halo work recomputed by a neighbouring CTA must not be counted twice): one
+// select per sum at the end instead of a branch per contribution.
 template <class Acc>
-struct GatedAcc {
-    Acc &acc;
-    bool on;
-    __device__ __forceinline__ void add(int r, double x)
+struct GatedAcc : Acc {
+    __device__ explicit GatedAcc(const double *jac) : Acc(jac) {}
+    __device__ __forceinline__ void into(Acc &acc, bool on)
     {
-        if (on)
-            acc.add(r, x);
+#pragma unroll
+        for (int r = 0; r < Acc::N; ++r)
+            acc.v[r] += on ? this->v[r] : 0.0;
     }
 };
 
@@ -272,19 +273,17 @@ template <class Acc>
 __device__ __forceinline__ void cs2_param_vjp(const Consts &k, const StageDev &st, double x, double y, double lam,
                                               Acc &par)
 {
-    if (k.eos != 2)
-        return;
     const double l = lam * k.inv_mach2;
+#pragma unroll
     for (int p = 0; p < 2; ++p) {
         const MassDev &m = st.m[p];
-        if (!(m.mass > 0.0))
-            continue;
+        const bool on = k.eos == 2 && m.mass > 0.0;
         const double dx = x - m.x, dy = y - m.y;
         const double s12 = crm::rsqrt_near(dx * dx + dy * dy + m.soft2);
         const double w = l * m.mass * s12 * s12 * s12;
-        par.add(5 * p + 0, w * dx);
-        par.add(5 * p + 1, w * dy);
-        par.add(5 * p + 4, l * s12);
+        par.add(5 * p + 0, on ? w * dx : 0.0);
+        par.add(5 * p + 1, on ? w * dy : 0.0);
+        par.add(5 * p + 4, on ? l * s12 : 0.0);
     }
 }
 
@@ -316,23 +315,10 @@ __device__ __forceinline__ void hlle_vjp(const double *pl, const double *pr, dou
         lap += w * (fl[q] - (ul[q] - ur[q]) * am - F);
         lam += w * (F - fr[q] - (ul[q] - ur[q]) * ap);
     }
-    double lvl = 0.0, lvr = 0.0, lcs = 0.0;
-    if (s_am == 1) {
-        lvl += lam;
-        lcs -= lam;
-    } else if (s_am == 2) {
-        lvr += lam;
-        lcs -= lam;
-    }
-    if (s_ap == 1) {
-        lvl += lap;
-        lcs += lap;
-    } else if (s_ap == 2) {
-        lvr += lap;
-        lcs += lap;
-    }
-    if (cs > 0.0)
-        *lcs2 += lcs * (0.5 * crm::recip_rn(cs));
+    double lvl = (s_am == 1 ? lam : 0.0) + (s_ap == 1 ? lap : 0.0);
+    double lvr = (s_am == 2 ? lam : 0.0) + (s_ap == 2 ? lap : 0.0);
+    const double lcs = (s_ap != 0 ? lap : 0.0) - (s_am != 0 ? lam : 0.0);
+    *lcs2 += cs > 0.0 ? lcs * (0.5 * crm::recip_rn(cs)) : 0.0;
     // fluxes: f0 = v u0, f1 = v u1 (+ rho cs2 if DIR == 0), f2 = v u2 (+ rho cs2 if DIR == 1)
     lvl += lfl[0] * ul[0] + lfl[1] * ul[1] + lfl[2] * ul[2];
     lvr += lfr[0] * ur[0] + lfr[1] * ur[1] + lfr[2] * ur[2];
@@ -498,9 +484,10 @@ __device__ __forceinline__ void rho_strain_of(const Consts &k, double rho, const
 // yy), and the adjoint of the zones' RK sums. Out, 8 doubles: lambda of
 // the minus-side face state (3), of the plus-side state (3), and of the
 // viscous flux's two rho * strain sums (2, the same for both sides).
+// Straight-line code (choices by selects), so that the march's two faces of a
+// row overlap in one thread.
 template <int DIR, class Acc>
-__device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, const MassT<double> *m,
-                                         const double *pL, const double *pR, const double *gL, const double *gR,
+__device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, const double *pL, const double *pR, const double *gL, const double *gR,
                                          const double *rL, const double *rR, const double *lul, const double *lur,
                                          double xf, double yf, Acc &par, double *o)
 {
@@ -512,7 +499,9 @@ __device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, co
         pr[q] = pR[q] - 0.5 * gR[q];
         lf[q] = (lur[q] - lul[q]) * cf;
     }
-    const double cs2 = cs2_generic(k, m, xf, yf), cs = crm::sqrt_rn(cs2);
+    const double cs2 = k.eos == 2 ? div_by<false>(-potential<false>(st.m, xf, yf), k.mach2, k.inv_mach2)
+                                  : (k.eos == 1 ? k.cs2 : 1.0);
+    const double cs = crm::sqrt_rn(cs2);
     double lpl[3] = {0, 0, 0}, lpr[3] = {0, 0, 0}, lcs2 = 0.0;
     hlle_vjp<DIR>(pl, pr, cs2, cs, hlle_select(pl[1 + DIR], pr[1 + DIR], cs), lf, lpl, lpr, &lcs2);
     cs2_param_vjp(k, st, xf, yf, lcs2, par);
@@ -520,13 +509,10 @@ __device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, co
         o[q] = lpl[q];
         o[3 + q] = lpr[q];
     }
-    if (k.nu > 0.0) {
-        o[6] = -hn * lf[1];
-        o[7] = -hn * lf[2];
-        par.add(10, -0.5 * (rL[0] + rR[0]) * lf[1] - 0.5 * (rL[1] + rR[1]) * lf[2]);
-    } else {
-        o[6] = o[7] = 0.0;
-    }
+    // without viscosity the products are zeros
+    o[6] = -hn * lf[1];
+    o[7] = -hn * lf[2];
+    par.add(10, k.nu > 0.0 ? -0.5 * (rL[0] + rR[0]) * lf[1] - 0.5 * (rL[1] + rR[1]) * lf[2] : 0.0);
 }
 
 // The adjoint gathered at one zone of [-1, ni] x [-1, nj] from its four
@@ -654,10 +640,10 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) adj_faces(Consts 
         const double *sl = a.sl + cl * 9, *sr = a.sl + cr * 9;
         double *o = (ydir ? a.fy : a.fx) + zi(i, j, nj) * 8;
         if (ydir)
-            face_vjp<1>(k, st, m, a.p + cl * 3, a.p + cr * 3, sl + 3, sr + 3, sl + 7, sr + 7, lul, lur,
+            face_vjp<1>(k, st, a.p + cl * 3, a.p + cr * 3, sl + 3, sr + 3, sl + 7, sr + 7, lul, lur,
                         k.xl + (i + 0.5) * k.dx, k.yl + (j + 0.0) * k.dy, par, o);
         else
-            face_vjp<0>(k, st, m, a.p + cl * 3, a.p + cr * 3, sl, sr, sl + 6, sr + 6, lul, lur,
+            face_vjp<0>(k, st, a.p + cl * 3, a.p + cr * 3, sl, sr, sl + 6, sr + 6, lul, lur,
                         k.xl + (i + 1.0) * k.dx, k.yl + (j + 0.5) * k.dy, par, o);
     }
     store_params<ADJ_THREADS, CHAIN>(a, par);
@@ -898,12 +884,13 @@ struct MarchSmem {
     double p[4][AM_NP][3];   // rows mod 4
     double sl[2][AM_NS][9];  // rows mod 2: gx (3), gy (3), rho * strain (3)
     double lr[2][AM_NS][3];  // RK-sum adjoint, rows mod 2
-    double yf[AM_NY][8];     // y-faces of the gathered row
+    double yf[AM_NY][9];     // y-faces of the gathered row (8 used: an odd stride keeps a warp's accesses in distinct banks)
     double lg[3][AM_NG][9];  // rows mod 3: lgx (3), lgy (3), lp (3)
     unsigned wd[4][AM_NS];   // limiter choices, rows mod 4
 };
 
-__device__ __forceinline__ int mod(int r, int m) { return ((r % m) + m) % m; }
+// ring slot of row r >= -16, m a constant
+__device__ __forceinline__ int mod(int r, int m) { return (int)((unsigned)(r + 48) % (unsigned)m); }
 
 // input_adjoint_at on the shared rings (row r must be in [r0 - 1 ..] of the
 // rings; c any padded column the strip covers)
@@ -988,8 +975,19 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
         }
     };
 
-    fetch(r_first - 6);
-    for (int r = r_first - 6; r <= r_last; ++r) {
+    // rows r_first - 3 and r_first - 2 straight into the ring: the first
+    // iteration stages row r_first - 1 and has slopes to compute
+    for (int c = t; c < 2 * AM_NP; c += AM_NT) {
+        const int L = r_first - 3 + c / AM_NP, col = c % AM_NP;
+        const bool live = L >= -2 && j0 - 3 + col >= -2 && j0 - 3 + col <= nj + 1;
+        const double *src = a.p + zi(L, j0 - 3 + col, nj) * 3;
+        double *d = sm.p[mod(L, 4)][col];
+        d[0] = live ? src[0] : 0.0;
+        d[1] = live ? src[1] : 0.0;
+        d[2] = live ? src[2] : 0.0;
+    }
+    fetch(r_first - 4);
+    for (int r = r_first - 4; r <= r_last; ++r) {
         // 1. stage the prefetched row, prefetch the next
         {
             const int L = r + 3, R = r + 2;
@@ -1052,10 +1050,11 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
                 const double *sA = sm.sl[mod(A, 2)][s], *sB = sm.sl[mod(A + 1, 2)][s];
                 // the face A + 1/2 belongs to the CTA owning row min(A + 1, ni - 1) and its column
                 const int orow = A + 1 < ni ? A + 1 : ni - 1;
-                GatedAcc<ParAcc<CHAIN>> gp{par, orow >= R0 && orow < R1 && cG >= j0 && cG < j0 + AM_BJ};
-                face_vjp<0>(k, st, m, sm.p[mod(A, 4)][pc], sm.p[mod(A + 1, 4)][pc], sA, sB, sA + 6, sB + 6,
+                GatedAcc<ParAcc<CHAIN>> gp(sh.jac);
+                face_vjp<0>(k, st, sm.p[mod(A, 4)][pc], sm.p[mod(A + 1, 4)][pc], sA, sB, sA + 6, sB + 6,
                             sm.lr[mod(A, 2)][s], sm.lr[mod(A + 1, 2)][s], k.xl + (A + 1.0) * k.dx,
                             k.yl + (cG + 0.5) * k.dy, gp, xnew);
+                gp.into(par, orow >= R0 && orow < R1 && cG >= j0 && cG < j0 + AM_BJ);
             }
             if (onY) {
                 double *o = sm.yf[t];
@@ -1065,10 +1064,11 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
                     const double *gL = sm.sl[mod(A, 2)][sl_], *gR = sm.sl[mod(A, 2)][sr_];
                     // the face j - 1/2 belongs to the CTA owning row A and column min(j, nj - 1)
                     const int ocol = j < nj ? j : nj - 1;
-                    GatedAcc<ParAcc<CHAIN>> gp{par, A >= R0 && A < R1 && ocol >= j0 && ocol < j0 + AM_BJ};
-                    face_vjp<1>(k, st, m, sm.p[mod(A, 4)][t + 1], sm.p[mod(A, 4)][t + 2], gL + 3, gR + 3, gL + 7,
+                    GatedAcc<ParAcc<CHAIN>> gp(sh.jac);
+                    face_vjp<1>(k, st, sm.p[mod(A, 4)][t + 1], sm.p[mod(A, 4)][t + 2], gL + 3, gR + 3, gL + 7,
                                 gR + 7, sm.lr[mod(A, 2)][sl_], sm.lr[mod(A, 2)][sr_], k.xl + (A + 0.5) * k.dx,
                                 k.yl + (j + 0.0) * k.dy, gp, o);
+                    gp.into(par, A >= R0 && A < R1 && ocol >= j0 && ocol < j0 + AM_BJ);
                 } else {
                     for (int q = 0; q < 8; ++q)
                         o[q] = 0.0;
@@ -1088,11 +1088,12 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
                     const bool own = interior && A >= R0 && A < R1 && cG >= j0 && cG < j0 + AM_BJ;
                     const size_t c = zi(A, cG, nj);
                     const double *sl = sm.sl[mod(A, 2)][t + 1];
-                    GatedAcc<ParAcc<CHAIN>> gp{par, own};
+                    GatedAcc<ParAcc<CHAIN>> gp(sh.jac);
                     zone_gather(k, st, A, cG, xnew, xprev, sm.yf[t], sm.yf[t + 1], sl, sl + 3,
                                 sm.p[mod(A, 4)][t + 2], sm.lr[mod(A, 2)][t + 1], interior,
                                 own && a.pn ? a.pn + c * 3 : nullptr, own && a.lam_n ? a.lam_n + c * 3 : nullptr,
                                 gp, g);
+                    gp.into(par, own);
                 } else {
                     for (int q = 0; q < 9; ++q)
                         g[q] = 0.0;
@@ -1338,7 +1339,7 @@ AdjArgs adj_args(const cbd_grid_t *grid, const void *stage_dev, void *workspace,
 // pass is the widest. Rows of the chained accumulator and of the per-block
 // partials.
 // shortest segment of the fused kernel's march
-constexpr int AM_MIN_ROWS = 4;
+constexpr int AM_MIN_ROWS = 1;
 
 int adj_rows(const cbd_grid_t *grid)
 {
@@ -1360,9 +1361,9 @@ int g_fused_adjoint = 1;
 // the fused kernel's segment length: 0 = by the wave rule of march_grid
 int g_march_rows = 0;
 
-// Strips of AM_BJ columns x segments of rows. A CTA marches its rows plus six
+// Strips of AM_BJ columns x segments of rows. A CTA marches its rows plus four
 // (the pipeline's lead rows), and CTAs run in waves of three per SM: the
-// segment length (4 .. 32 rows) minimises waves x (rows + 6), the longer
+// segment length (1 .. 32 rows) minimises waves x (rows + 4), the longer
 // segment on a tie.
 dim3 march_grid(int ni, int nj)
 {
@@ -1378,7 +1379,7 @@ dim3 march_grid(int ni, int nj)
     long best_cost = -1;
     for (int rows = 32; rows >= AM_MIN_ROWS; --rows) {
         const long ctas = (long)strips * ((ni + rows - 1) / rows);
-        const long cost = (ctas + slots - 1) / slots * (rows + 6);
+        const long cost = (ctas + slots - 1) / slots * (rows + 4);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = rows;
@@ -1586,7 +1587,7 @@ int cbdiso_b200_set_adjoint_variant(int fused)
 
 int cbdiso_b200_set_adjoint_segment_rows(int rows)
 {
-    if (rows != 0 && (rows < AM_MIN_ROWS || rows > 32))
+    if (rows != 0 && (rows < 4 || rows > 32))
         return CBD_ERR_ARGUMENT;
     g_march_rows = rows;
     return CBD_OK;
