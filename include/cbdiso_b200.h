@@ -459,6 +459,13 @@ int cbdiso_b200_reduce(
     const cbd_grid_t *grid, const cbd_epilogue_t *epilogue, const double *primitive,
     double *scratch, double *result, void *stream);
 
+/* `bytes` of device memory at `src` to the host memory at `dst`, behind the
+ * work queued on `stream`; returns when they have arrived. */
+int cbdiso_b200_read(void *dst, const void *src, size_t bytes, void *stream);
+
+/* Zeros `bytes` of device memory, in stream order. */
+int cbdiso_b200_clear(void *dst, size_t bytes, void *stream);
+
 /* Test hook (no counterpart in the reference): evaluates the correctly
  * rounded arithmetic the EXACT stencil is built from, on device arrays of n
  * elements: out[4i] = a/b, out[4i+1] = a^-1.5, out[4i+2] = a^4,

@@ -39,6 +39,18 @@ class CbdError(RuntimeError):
         super().__init__(f"{where}: {STATUS.get(status, 'unknown status')} (status {status})")
 
 
+def current_stream():
+    """Handle of the current device's current torch stream (an int). The raw
+    accessor takes a fraction of a microsecond where building a Stream object
+    takes four, several times a step."""
+    import torch
+
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
+
+
 class Mass(Structure):
     _fields_ = [("x", c_double), ("y", c_double), ("vx", c_double), ("vy", c_double), ("mass", c_double),
                 ("softening_length", c_double), ("sink_rate", c_double), ("sink_radius", c_double),
@@ -133,6 +145,10 @@ def _declare(lib):
     lib.cbdiso_b200_stage_record.restype = c_int
     lib.cbdiso_b200_eval_primitives.argtypes = [ctypes.c_long, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.cbdiso_b200_eval_primitives.restype = c_int
+    lib.cbdiso_b200_read.argtypes = [c_void_p, c_void_p, c_size_t, c_void_p]
+    lib.cbdiso_b200_read.restype = c_int
+    lib.cbdiso_b200_clear.argtypes = [c_void_p, c_size_t, c_void_p]
+    lib.cbdiso_b200_clear.restype = c_int
     lib.cbdiso_b200_eval_roots.argtypes = [ctypes.c_long, c_void_p, c_void_p, c_void_p, c_void_p]
     lib.cbdiso_b200_eval_roots.restype = c_int
     lib.cbdiso_b200_stepper_bytes.argtypes = []
@@ -248,7 +264,7 @@ def exported_symbols():
         "cbdiso_b200_status_string", "cbdiso_b200_version", "cbdiso_b200_scratch_bytes", "cbdiso_b200_fill_guards",
         "cbdiso_b200_advance_stage", "cbdiso_b200_reduce", "cbdiso_b200_abi_sizes",
         "cbdiso_b200_stage_record_bytes", "cbdiso_b200_stage_record", "cbdiso_b200_eval_primitives",
-        "cbdiso_b200_eval_roots",
+        "cbdiso_b200_eval_roots", "cbdiso_b200_read", "cbdiso_b200_clear",
         "cbdiso_b200_advance_stage_noalloc", "cbdiso_b200_face_cache_bytes", "cbdiso_b200_advance_stage_cached",
         "cbdiso_b200_stepper_bytes", "cbdiso_b200_stepper_init",
         "cbdiso_b200_step_prologue", "cbdiso_b200_batch_disk_bytes", "cbdiso_b200_batch_disk_record",

@@ -33,9 +33,9 @@ from typing import NamedTuple
 import numpy as np
 
 from . import _capi, _hostio
-from .cbdiso_2d import _as_diagnostic, _diag_struct, _mass_struct
+from .cbdiso_2d import MassStructs, _as_diagnostic, _diag_struct
 from .mesh import is_planar_cartesian_2d
-from .physics import MassCache, Physics, enum_value
+from .physics import Physics, enum_value
 from .solver_base import SolverBase
 
 logger = getLogger(__name__)
@@ -193,9 +193,14 @@ class Solver(SolverBase):
             self._fcache[:32].zero_()
         # the wavespeed maximum of the current state (slot 0; the multi-GPU
         # solver all-reduces it in place) and, apart, the diagnostic sums
-        self._result = torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, **f64)
+        # of either of two blocks in turn: a step's second stage needs its slot
+        # zeroed, and the one it will use is cleared a step ahead, while nobody
+        # waits for the launches
+        self._results = [torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, **f64) for _ in range(2)]
+        self._result = self._results[0]
         self._sums = torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, **f64)
         self._result_host = torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, dtype=torch.float64).pin_memory()
+        self._result_np = self._result_host.numpy()
         self._ws_valid = False
         self._time = float(time)
         self.h2d_bytes = 0
@@ -207,13 +212,11 @@ class Solver(SolverBase):
 
     @staticmethod
     def _ptr(t):
-        return ctypes.c_void_p(t.data_ptr())
+        return t.data_ptr()
 
     @staticmethod
     def _stream():
-        import torch
-
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _capi.current_stream()
 
     @staticmethod
     def _check(status, where):
@@ -221,10 +224,7 @@ class Solver(SolverBase):
 
     def _stage(self, time, a, dt):
         st = _capi.GamStage()
-        m1, m2 = self._point_masses(time)
-        _mass_struct(m1, st.mass[0])
-        _mass_struct(m2, st.mass[1])
-        st.buffer_central_mass = m1.mass + m2.mass
+        st.mass, st.buffer_central_mass = self._mass_pair(time)
         st.a, st.dt = a, dt
         return st
 
@@ -248,28 +248,29 @@ class Solver(SolverBase):
                    for x, y in zip(a.mass, b.mass))
 
     def _point_masses(self, t):
+        return self._masses().masses(t)
+
+    def _mass_pair(self, t):
+        return self._masses()(t)
+
+    def _masses(self):
         masses = self.__dict__.get("_mass_cache")
         if masses is None or masses.physics is not self._physics:
-            masses = self._mass_cache = MassCache(self._physics)
-        return masses(t)
+            masses = self._mass_cache = MassStructs(self._physics)
+        return masses
 
     def _read(self, n, source=None):
-        import torch
-
         source = self._result if source is None else source
-        self._result_host[:n].copy_(source[:n], non_blocking=True)
-        torch.cuda.current_stream().synchronize()
+        self._check(self._lib.cbdiso_b200_read(self._result_host.data_ptr(), source.data_ptr(), 8 * n,
+                                               self._stream()), "read result")
         self.d2h_bytes += 8 * n
-        return self._result_host[:n].numpy().copy()
+        return self._result_np[:n].copy()
 
     def _reduce(self, diags):
         """The sums of `diags` (at most 4) on the current state into
         self._sums; with no diagnostics, the wavespeed maximum into
         self._result."""
-        masses = (_capi.Mass * 2)()
-        m1, m2 = self._point_masses(self._time)
-        _mass_struct(m1, masses[0])
-        _mass_struct(m2, masses[1])
+        masses, _ = self._mass_pair(self._time)
         structs = (_capi.Diag * max(1, len(diags)))()
         for k, d in enumerate(diags):
             _diag_struct(d, structs[k])
@@ -328,17 +329,18 @@ class Solver(SolverBase):
         """One RK2 step (cbdgam_2d.py:473-489): two stage kernels, masses at
         each stage's start time, the stage times as the reference updates
         them."""
+        import torch
+
         dt = float(dt)
         if not math.isfinite(dt):
             raise _capi.CbdError(_capi.NONFINITE, "advance: time step")
-        lib, g = self._lib, self._grid
+        lib = self._lib
         stream = self._stream()
         t0 = self._time
         t1 = t0 * 0.0 + (t0 + dt) * (1.0 - 0.0)
         t2 = t0 * 0.5 + (t1 + dt) * (1.0 - 0.5)
         a_buf, b_buf = self._buf
         s1 = self._stage(t0, 0.0, dt)
-        self._result[:1].zero_()
         self._launch(s1, a_buf, None, b_buf, None, 2, stream)
         if self._stage_hook is not None:
             self._stage_hook(0, b_buf)
@@ -346,7 +348,13 @@ class Solver(SolverBase):
         # fills the face cache when its masses are the step's end masses
         s2 = self._stage(t1, 0.5, dt)
         writer = self._same_masses(s2, self._stage(t2, 0.5, dt))
-        self._launch(s2, b_buf, a_buf, a_buf, self._result, 1 if writer else 0, stream)
+        old, new = self._result, self._results[1 if self._result is self._results[0] else 0]
+        if torch.cuda.is_current_stream_capturing():
+            # a captured step may be replayed alone: it clears its own slot
+            self._check(lib.cbdiso_b200_clear(new.data_ptr(), 8, stream), "clear")
+        self._launch(s2, b_buf, a_buf, a_buf, new, 1 if writer else 0, stream)
+        self._result = new
+        self._check(lib.cbdiso_b200_clear(old.data_ptr(), 8, stream), "clear")
         if self._stage_hook is not None:
             self._stage_hook(1, a_buf)
         self._time = t2

@@ -109,6 +109,31 @@ def _mass_struct(m, out):
     out.sink_model = enum_value(m.sink_model)
 
 
+class MassStructs:
+    """The ctypes records of physics.point_masses(t), with their total mass,
+    for the last few times t (physics.MassCache, as the library takes them)."""
+
+    def __init__(self, physics, size=4):
+        self.physics = physics
+        self.masses = MassCache(physics, size)
+        self.size = size
+        self.entries = []
+
+    def __call__(self, t):
+        for tc, pair, total in self.entries:
+            if tc == t:
+                return pair, total
+        m1, m2 = self.masses(t)
+        pair = (_capi.Mass * 2)()
+        _mass_struct(m1, pair[0])
+        _mass_struct(m2, pair[1])
+        total = m1.mass + m2.mass
+        self.entries.append((t, pair, total))
+        if len(self.entries) > self.size:
+            self.entries.pop(0)
+        return pair, total
+
+
 def _diag_struct(d: Diagnostic, out):
     out.quantity = _capi.QUANTITY[d.quantity]
     wm = d.which_mass
@@ -245,6 +270,8 @@ class Solver(SolverBase):
             self._fcache[:32].zero_()
         self._result = torch.zeros(1 + 2 * _capi.MAX_DIAG, **f64)
         self._result_host = torch.zeros(1 + 2 * _capi.MAX_DIAG, dtype=torch.float64).pin_memory()
+        self._result_np = self._result_host.numpy()
+        self._epilogue_base = None  # the epilogue record of this solver's diagnostics, less its masses
 
         # stage records: a small ring of pinned host slots, one device block
         self._rec_bytes = int(self._lib.cbdiso_b200_stage_record_bytes())
@@ -268,37 +295,37 @@ class Solver(SolverBase):
 
     @staticmethod
     def _ptr(t):
-        return ctypes.c_void_p(t.data_ptr())
+        return t.data_ptr()
 
     @staticmethod
     def _stream():
-        import torch
-
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _capi.current_stream()
 
     def _check(self, status, where):
         _capi.check(status, where)
 
     def _epilogue(self, time, want_ws, diags):
-        ep = _capi.Epilogue()
-        m1, m2 = self._point_masses(time)
-        _mass_struct(m1, ep.mass[0])
-        _mass_struct(m2, ep.mass[1])
+        own = diags is self._device_diags
+        if own and self._epilogue_base is not None:
+            ep = _capi.Epilogue.from_buffer_copy(self._epilogue_base)
+        else:
+            ep = _capi.Epilogue()
+            ep.num_diag = len(diags)
+            for k, d in enumerate(diags):
+                _diag_struct(d, ep.diag[k])
+            if own:
+                self._epilogue_base = _capi.Epilogue.from_buffer_copy(ep)
         ep.want_wavespeed = int(want_ws)
-        ep.num_diag = len(diags)
-        for k, d in enumerate(diags):
-            _diag_struct(d, ep.diag[k])
+        ep.mass = self._mass_pair(time)[0]
         return ep
 
     def _read_result(self):
-        import torch
-
         if self._cached is None:
             n = 1 + 2 * len(self._device_diags)
-            self._result_host[:n].copy_(self._result[:n], non_blocking=True)
-            torch.cuda.current_stream().synchronize()
+            self._check(self._lib.cbdiso_b200_read(self._result_host.data_ptr(), self._result.data_ptr(), 8 * n,
+                                                   self._stream()), "read result")
             self.d2h_bytes += 8 * n
-            self._cached = self._result_host[:n].numpy().copy()
+            self._cached = self._result_np[:n].copy()
         return self._cached
 
     def _reduce_now(self, want_ws, diags):
@@ -360,10 +387,10 @@ class Solver(SolverBase):
         previous step's end) are set, its record carried by the launch's own
         parameters, so that the device idles as little as possible between
         the caller's wavespeed read and this step; the later stages' orbits
-        and records are built on the host while it runs and reach the device
-        as one copy ahead of their launches."""
-        import torch
-
+        and records are built on the host while it runs. The last stage's
+        record, with the epilogue's masses, goes as launch parameters too; a
+        stage between the two (RK3) reads the end-of-step masses from a record
+        copied to the device."""
         dt = float(dt)
         if not math.isfinite(dt):
             raise _capi.CbdError(_capi.NONFINITE, "advance: time step")
@@ -385,12 +412,9 @@ class Solver(SolverBase):
 
         def stage(s):
             st = _capi.Stage()
-            m1, m2 = self._point_masses(times[s])
-            _mass_struct(m1, st.mass[0])
-            _mass_struct(m2, st.mass[1])
+            st.mass, st.buffer_central_mass = self._mass_pair(times[s])
             st.a = weights[s]
             st.dt = dt
-            st.buffer_central_mass = m1.mass + m2.mass
             return st
 
         last = len(weights) - 1
@@ -400,24 +424,29 @@ class Solver(SolverBase):
         self._launch_stage(0, plan, weights, epilogue, stream, stage=stage(0))
         rb = self._rec_bytes
         if last > 0:
-            # the later stages' records: a slot of the pinned ring whose
+            epilogue = self._epilogue(time_end, True, diags)
+        if last > 1:
+            import torch
+
+            # the middle stages' records: a slot of the pinned ring whose
             # previous copy has completed, then one copy to the device
             slot = self._ring_next
             self._ring_next = (slot + 1) % len(self._ring)
             if self._ring_events[slot] is not None:
                 self._ring_events[slot].synchronize()
             host = self._ring[slot]
-            epilogue = self._epilogue(time_end, True, diags)
-            for s in range(1, last + 1):
+            for s in range(1, last):
                 self._check(lib.cbdiso_b200_stage_record(ctypes.byref(g), ctypes.byref(stage(s)),
                                                          ctypes.byref(epilogue),
                                                          ctypes.c_void_p(host.data_ptr() + s * rb)), "stage_record")
-            self._records[rb:].copy_(host[rb:], non_blocking=True)
+            self._records[rb:last * rb].copy_(host[rb:last * rb], non_blocking=True)
             ev = torch.cuda.Event()
             ev.record()
             self._ring_events[slot] = ev
-            for s in range(1, last + 1):
-                self._launch_stage(s, plan, weights, epilogue if s == last else None, stream)
+            for s in range(1, last):
+                self._launch_stage(s, plan, weights, None, stream)
+        if last > 0:
+            self._launch_stage(last, plan, weights, epilogue, stream, stage=stage(last))
         self.h2d_bytes += len(weights) * rb  # every stage's record: launch parameters or the copy
         self._finish_stages(len(weights), None)
         self._time = time_end
@@ -427,7 +456,13 @@ class Solver(SolverBase):
     def _point_masses(self, t):
         masses = self.__dict__.get("_mass_cache")
         if masses is None or masses.physics is not self._physics:
-            masses = self._mass_cache = MassCache(self._physics)
+            masses = self._mass_cache = MassStructs(self._physics)
+        return masses.masses(t)
+
+    def _mass_pair(self, t):
+        masses = self.__dict__.get("_mass_cache")
+        if masses is None or masses.physics is not self._physics:
+            masses = self._mass_cache = MassStructs(self._physics)
         return masses(t)
 
     # ------------------------------------------------------------------
@@ -738,10 +773,10 @@ class Solver(SolverBase):
             rec = ctypes.c_void_p(self._records.data_ptr() + s * self._rec_bytes)
         else:
             rec = None
-        common = (ctypes.byref(self._grid), ctypes.byref(stage), rec, self._ptr(rd),
-                  self._ptr(pn) if pn is not None else None, self._ptr(wr),
-                  ctypes.byref(epilogue) if epilogue is not None else None, self._ptr(self._scratch),
-                  self._ptr(self._result))
+        common = (ctypes.byref(self._grid), ctypes.byref(stage), rec, rd.data_ptr(),
+                  pn.data_ptr() if pn is not None else None, wr.data_ptr(),
+                  ctypes.byref(epilogue) if epilogue is not None else None, self._scratch.data_ptr(),
+                  self._result.data_ptr())
         role = self._cache_role(s, len(weights))
         if role:
             status = self._lib.cbdiso_b200_advance_stage_cached(*common, self._ptr(self._fcache), role, stream)

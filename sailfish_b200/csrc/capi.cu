@@ -577,6 +577,22 @@ int cbdiso_b200_reduce(
     return CBD_OK;
 }
 
+int cbdiso_b200_read(void *dst, const void *src, size_t bytes, void *stream)
+{
+    if (!dst || !src)
+        return CBD_ERR_ARGUMENT;
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    return status_of(e == cudaSuccess ? cudaStreamSynchronize(s) : e);
+}
+
+int cbdiso_b200_clear(void *dst, size_t bytes, void *stream)
+{
+    if (!dst)
+        return CBD_ERR_ARGUMENT;
+    return status_of(cudaMemsetAsync(dst, 0, bytes, static_cast<cudaStream_t>(stream)));
+}
+
 int cbdiso_b200_eval_primitives(long n, const double *a, const double *b, double *out, void *stream)
 {
     if (n < 0 || (n > 0 && (!a || !b || !out)))
