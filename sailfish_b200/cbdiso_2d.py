@@ -273,12 +273,9 @@ class Solver(SolverBase):
         self._result_np = self._result_host.numpy()
         self._epilogue_base = None  # the epilogue record of this solver's diagnostics, less its masses
 
-        # stage records: a small ring of pinned host slots, one device block
+        # stage records as the device stepper writes them
         self._rec_bytes = int(self._lib.cbdiso_b200_stage_record_bytes())
         nstage = len(RK_WEIGHTS[options.rk_order])
-        self._ring = [torch.zeros(nstage * self._rec_bytes, dtype=torch.uint8).pin_memory() for _ in range(4)]
-        self._ring_events = [None] * len(self._ring)
-        self._ring_next = 0
         self._records = torch.zeros(nstage * self._rec_bytes, dtype=torch.uint8, device=self.device)
 
         self._device_diags = [d for d in physics.diagnostics if d.quantity != "time"]
@@ -387,16 +384,13 @@ class Solver(SolverBase):
         previous step's end) are set, its record carried by the launch's own
         parameters, so that the device idles as little as possible between
         the caller's wavespeed read and this step; the later stages' orbits
-        and records are built on the host while it runs. The last stage's
-        record, with the epilogue's masses, goes as launch parameters too; a
-        stage between the two (RK3) reads the end-of-step masses from a record
-        copied to the device."""
+        and records are built on the host while it runs and go as launch
+        parameters too."""
         dt = float(dt)
         if not math.isfinite(dt):
             raise _capi.CbdError(_capi.NONFINITE, "advance: time step")
         weights = RK_WEIGHTS[self._options.rk_order]
         time0 = self._time
-        lib, g = self._lib, self._grid
         stream = self._stream()
 
         # stage times follow cbdiso_2d.py:239 exactly
@@ -418,36 +412,15 @@ class Solver(SolverBase):
             return st
 
         last = len(weights) - 1
-        # the first stage, its record as launch parameters; without an
-        # epilogue (RK2, RK3) its record's end-of-step masses are never read
+        # without an epilogue the first stage's record's end-of-step masses are
+        # never read; a middle stage (RK3) compares its masses with them and
+        # takes them from an epilogue record that asks for nothing
         epilogue = self._epilogue(time_end, True, diags) if last == 0 else None
         self._launch_stage(0, plan, weights, epilogue, stream, stage=stage(0))
-        rb = self._rec_bytes
-        if last > 0:
-            epilogue = self._epilogue(time_end, True, diags)
-        if last > 1:
-            import torch
-
-            # the middle stages' records: a slot of the pinned ring whose
-            # previous copy has completed, then one copy to the device
-            slot = self._ring_next
-            self._ring_next = (slot + 1) % len(self._ring)
-            if self._ring_events[slot] is not None:
-                self._ring_events[slot].synchronize()
-            host = self._ring[slot]
-            for s in range(1, last):
-                self._check(lib.cbdiso_b200_stage_record(ctypes.byref(g), ctypes.byref(stage(s)),
-                                                         ctypes.byref(epilogue),
-                                                         ctypes.c_void_p(host.data_ptr() + s * rb)), "stage_record")
-            self._records[rb:last * rb].copy_(host[rb:last * rb], non_blocking=True)
-            ev = torch.cuda.Event()
-            ev.record()
-            self._ring_events[slot] = ev
-            for s in range(1, last):
-                self._launch_stage(s, plan, weights, None, stream)
-        if last > 0:
-            self._launch_stage(last, plan, weights, epilogue, stream, stage=stage(last))
-        self.h2d_bytes += len(weights) * rb  # every stage's record: launch parameters or the copy
+        for s in range(1, last + 1):
+            epilogue = self._epilogue(time_end, True, diags) if s == last else self._epilogue(time_end, False, [])
+            self._launch_stage(s, plan, weights, epilogue, stream, stage=stage(s))
+        self.h2d_bytes += len(weights) * self._rec_bytes  # every stage's record, as launch parameters
         self._finish_stages(len(weights), None)
         self._time = time_end
         self._cached = None
