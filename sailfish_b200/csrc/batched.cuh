@@ -116,16 +116,16 @@ __global__ void __launch_bounds__(BJ, MINB) batched_stage_kernel(const BatchArgs
         } else if (ROLE == ROLE_WRITER) {
             // the same answer in every thread; the block with the disk's first tile writes the key
             const bool store = cached && cache_write_check<PREC>(k, st, sa.fcache, u == D.unit_begin);
-            march_tile<BJ, FAST, CACHE_WRITE, false>(k, st, sa, c0, D.strip_width, r0, store);
+            march_tile<BJ, FAST, CACHE_WRITE>(k, st, sa, c0, D.strip_width, r0, store);
         } else if (ROLE == ROLE_READER) {
             if (cached) {
-                march_tile<BJ, FAST, CACHE_READ, false>(k, st, sa, c0, D.strip_width, r0);
+                march_tile<BJ, FAST, CACHE_READ>(k, st, sa, c0, D.strip_width, r0);
                 // the fill kernel ran before this launch; no tile reads the key
                 if (u == D.unit_begin)
                     cache_write_key<PREC>(k, st, sa.fcache);
             }
         } else {
-            march_tile<BJ, FAST, CACHE_NONE, false>(k, st, sa, c0, D.strip_width, r0);
+            march_tile<BJ, FAST, CACHE_NONE>(k, st, sa, c0, D.strip_width, r0);
         }
         __syncthreads();
     }
