@@ -165,19 +165,25 @@ int cbd::segment_rows(int ni, int strips, int bj, int slots)
 namespace {
 
 // Launch shape of the stage kernel. Defaults: 256-column strips (3 resident
-// CTAs per SM) on grids of at least 2048^2 zones, 128-column strips compiled
-// for 6 resident CTAs per SM below that (64-column strips and 12 CTAs for
-// narrow grids), and rows per CTA chosen for whole waves (below). (Measured
-// per step at 32 and 16 rows: 4096^2 2.188 -> 2.157 ms and 2048^2 0.657 ->
-// 0.637 ms with 256 columns; 1024^2 0.232 -> 0.234 ms.)
+// CTAs per SM) on grids of at least 900^2 zones, 128-column strips compiled
+// for 5 resident CTAs per SM below that, and rows per CTA by segment_rows.
+// Measured, us per step, 256 columns / 128 at 5 CTAs / 128 at 6 (rows by the
+// rule each time): 256^2 - / 33.0 / 33.9, 512^2 60.1 / 59.2 / 60.4, 768^2
+// 93.0 / 92.5 / 95.5, 900^2 133 / 135 / 143, 1024^2 147 / 158 / 158, 1200^2
+// 196 / 211 / 213, 1511^2 286 / 301 / 306, 2048^2 477 / 509 / 495, 3000^2 965 /
+// 975 / 1006; up to 128 columns, 128-column strips at 5 / 64 at 12: 16^2 23.3 /
+// 24.8, 64^2 25.8 / 27.1, 96^2 25.9 / 27.3. Long grids of at most 64 columns
+// keep 64-column strips (10 CTAs): 4096 x 64 66 against 72, 16384 x 64 175
+// against 211 (4096 x 32 60 against 56).
 LaunchShape stage_shape(int ni, int nj, int bj, int rows, int occupancy = 0)
 {
     const bool chosen = rows <= 0;
     LaunchShape s;
     if (bj != 64 && bj != 128 && bj != 256) {
-        bj = nj >= 2048 && (long)ni * nj >= 2048L * 2048 ? 256 : (nj > 96 ? 128 : 64);
+        const long zones = (long)ni * nj;
+        bj = nj >= 900 && zones >= 900L * 900 ? 256 : (nj <= 64 && zones >= 4096L * 48 ? 64 : 128);
         if (occupancy == 0)
-            occupancy = bj == 128 ? 6 : 12;
+            occupancy = bj == 128 ? 5 : 10;
     }
     s.minb = 1;
     // 256-column strips: 3 CTAs per SM (80 registers, 68 KB of shared memory each)
