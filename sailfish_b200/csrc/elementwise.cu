@@ -4,6 +4,7 @@
 // arithmetic matches the reference's CPU build operation for operation.
 #include "cbd_internal.h"
 #include "elementwise.h"
+#include "zone_walk.cuh"
 
 namespace cbd {
 
@@ -17,9 +18,12 @@ __device__ __forceinline__ size_t zoff(int i, int j, int nj)
 // Threads map to zones with j (the contiguous axis) fastest.
 __global__ void p2c_kernel(int ni, int nj, const double *p, double *u)
 {
+    chain_begin();
     const long n = (long)ni * nj;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < n; z += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(z / nj), j = (int)(z - (long)i * nj);
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    ZoneWalk w(z0, step, nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const size_t o = zoff(i, j, nj);
         const double rho = p[o];
         u[o] = rho;
@@ -31,9 +35,12 @@ __global__ void p2c_kernel(int ni, int nj, const double *p, double *u)
 __global__ void source_kernel(int ni, int nj, double xl, double yl, double dx, double dy, MassDev m,
                               const double *p, double *rate)
 {
+    chain_begin();
     const long n = (long)ni * nj;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < n; z += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(z / nj), j = (int)(z - (long)i * nj);
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    ZoneWalk w(z0, step, nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const size_t o = zoff(i, j, nj);
         const double xc = xl + (i + 0.5) * dx;
         const double yc = yl + (j + 0.5) * dy;
@@ -47,10 +54,13 @@ __global__ void source_kernel(int ni, int nj, double xl, double yl, double dx, d
 
 __global__ void wavespeed_kernel(int ni, int nj, Consts k, MassDev m0, MassDev m1, const double *p, double *ws)
 {
+    chain_begin();
     const long n = (long)ni * nj;
     MassDev m[2] = {m0, m1};
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < n; z += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(z / nj), j = (int)(z - (long)i * nj);
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    ZoneWalk w(z0, step, nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const double xc = k.xl + (i + 0.5) * k.dx;
         const double yc = k.yl + (j + 0.5) * k.dy;
         const double c2 = sound_speed2<false>(k, m, xc, yc);
@@ -61,8 +71,10 @@ __global__ void wavespeed_kernel(int ni, int nj, Consts k, MassDev m0, MassDev m
 __global__ void fill_guards_kernel(int ni, int nj, double *p)
 {
     const long wi = ni + 2 * NG, wj = nj + 2 * NG;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < wi * wj; z += (long)gridDim.x * blockDim.x) {
-        const int ii = (int)(z / wj) - NG, jj = (int)(z % wj) - NG;
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    ZoneWalk w(z0, step, (int)wj);
+    for (long z = z0; z < wi * wj; z += step, w.next()) {
+        const int ii = w.i - NG, jj = w.j - NG;
         if (ii >= 0 && ii < ni && jj >= 0 && jj < nj)
             continue;
         const int ci = ii < 0 ? 0 : (ii >= ni ? ni - 1 : ii);
@@ -85,8 +97,10 @@ __global__ void __launch_bounds__(BJ) reduce_kernel(const Consts k, const StageD
     for (int v = 0; v < PARTIAL_STRIDE; ++v)
         acc[v] = 0.0;
     const long n = (long)k.ni * k.nj;
-    for (long z = blockIdx.x * (long)BJ + threadIdx.x; z < n; z += (long)gridDim.x * BJ) {
-        const int i = (int)(z / k.nj), j = (int)(z - (long)i * k.nj);
+    const long step = (long)gridDim.x * BJ, z0 = blockIdx.x * (long)BJ + threadIdx.x;
+    ZoneWalk w(z0, step, k.nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const double *pc = p + zoff(i, j, k.nj);
         const double pz[3] = {pc[0], pc[1], pc[2]};
         const double xc = k.xl + (i + 0.5) * k.dx;
@@ -134,22 +148,21 @@ inline int blocks_for(long n, int bs, int cap)
 
 cudaError_t launch_p2c(int ni, int nj, const double *p, double *u, cudaStream_t s)
 {
-    p2c_kernel<<<blocks_for((long)ni * nj, 256, 148 * 16), 256, 0, s>>>(ni, nj, p, u);
-    return cudaGetLastError();
+    return launch_chained(p2c_kernel, blocks_for((long)ni * nj, 256, 148 * 16), 256, 0, s, ni, nj, p, u);
 }
 
 cudaError_t launch_source(int ni, int nj, double xl, double yl, double dx, double dy, const MassDev &m,
                           const double *p, double *rate, cudaStream_t s)
 {
-    source_kernel<<<blocks_for((long)ni * nj, 256, 148 * 16), 256, 0, s>>>(ni, nj, xl, yl, dx, dy, m, p, rate);
-    return cudaGetLastError();
+    return launch_chained(source_kernel, blocks_for((long)ni * nj, 256, 148 * 16), 256, 0, s, ni, nj, xl, yl, dx, dy, m,
+                          p, rate);
 }
 
 cudaError_t launch_wavespeed(const Consts &k, const MassDev &m0, const MassDev &m1, const double *p, double *ws,
                              cudaStream_t s)
 {
-    wavespeed_kernel<<<blocks_for((long)k.ni * k.nj, 256, 148 * 16), 256, 0, s>>>(k.ni, k.nj, k, m0, m1, p, ws);
-    return cudaGetLastError();
+    return launch_chained(wavespeed_kernel, blocks_for((long)k.ni * k.nj, 256, 148 * 16), 256, 0, s, k.ni, k.nj, k, m0,
+                          m1, p, ws);
 }
 
 cudaError_t launch_fill_guards(int ni, int nj, double *p, cudaStream_t s)

@@ -22,6 +22,7 @@
 #include "cbdiso_b200.h"
 #include "chain.cuh"
 #include "cr_math.cuh"
+#include "zone_walk.cuh"
 
 namespace cbd {
 cudaStream_t drop_in_stream();  // capi.cu: the stream set by cbdiso_b200_set_stream
@@ -392,8 +393,10 @@ __global__ void __launch_bounds__(128) cache_fill_kernel(Consts k, Stage st, dou
 __global__ void p2c_kernel(int ni, int nj, double gamma, const double *prim, double *cons)
 {
     const long n = (long)ni * nj;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < n; z += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(z / nj), j = (int)(z % nj);
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    cbd::ZoneWalk w(z0, step, nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         prim_to_cons(prim + at(i, j, nj), cons + at(i, j, nj), gamma);
     }
 }
@@ -401,8 +404,10 @@ __global__ void p2c_kernel(int ni, int nj, double gamma, const double *prim, dou
 __global__ void wavespeed_kernel(int ni, int nj, double gamma, const double *prim, double *ws)
 {
     const long n = (long)ni * nj;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < n; z += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(z / nj), j = (int)(z % nj);
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    cbd::ZoneWalk w(z0, step, nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const double *p = prim + at(i, j, nj);
         ws[(size_t)(i + NG) * (nj + 2 * NG) + (j + NG)] = max_wavespeed(p, cs2_of(gamma, p));
     }
@@ -415,8 +420,10 @@ __global__ void source_kernel(int ni, int nj, double xl, double yl, double dx, d
     const Mass ms[2] = {m1, m2};
     const bool massless = m1.mass == 0.0 && m2.mass == 0.0;
     const long n = (long)ni * nj;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < n; z += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(z / nj), j = (int)(z % nj);
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    cbd::ZoneWalk w(z0, step, nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const double xc = xl + (i + 0.5) * dx, yc = yl + (j + 0.5) * dy;
         const double *p = prim + at(i, j, nj);
         const double T = p[3] / p[0];
@@ -429,8 +436,10 @@ __global__ void source_kernel(int ni, int nj, double xl, double yl, double dx, d
 __global__ void guards_kernel(int ni, int nj, double *a)
 {
     const long wi = ni + 2 * NG, wj = nj + 2 * NG;
-    for (long z = blockIdx.x * (long)blockDim.x + threadIdx.x; z < wi * wj; z += (long)gridDim.x * blockDim.x) {
-        const int ii = (int)(z / wj) - NG, jj = (int)(z % wj) - NG;
+    const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    cbd::ZoneWalk w(z0, step, (int)wj);
+    for (long z = z0; z < wi * wj; z += step, w.next()) {
+        const int ii = w.i - NG, jj = w.j - NG;
         if (ii >= 0 && ii < ni && jj >= 0 && jj < nj)
             continue;
         const int ci = ii < 0 ? 0 : (ii >= ni ? ni - 1 : ii);
@@ -468,22 +477,36 @@ struct RedArgs {
 __device__ __forceinline__ void diag_rates(const RedArgs &r, const Diag &d, int which, double xc, double yc,
                                            const double *p, double *rate)
 {
-    Mass ms[2] = {r.m[0], r.m[1]};
-    const double gravity = d.accretion ? 0.0 : 1.0, accretion = d.accretion ? 1.0 : 0.0;
-    for (int k = 0; k < 2; ++k) {
-        ms[k].mass = ms[k].mass * gravity;
-        ms[k].rate = ms[k].rate * accretion;
+    Mass m = r.m[which - 1];
+    const double T = div_rn(p[3], p[0]);
+    double h = 1.0;
+    if (d.accretion) {
+        // without masses every height is 1; beyond the sink's reach the rates are
+        // zeros (of Sigma and the velocity, so that a NaN still shows)
+        const double dx = xc - m.x, dy = yc - m.y;
+        if (dx * dx + dy * dy > 16.0 * (m.radius * m.radius) * (1.0 + 1e-10)) {
+            rate[0] = -(p[0] * 0.0);
+            rate[1] = rate[0] * p[1];
+            rate[2] = rate[0] * p[2];
+            rate[3] = 0.0;
+            return;
+        }
+        m.mass = m.mass * 0.0;
+    } else {
+        m.rate = m.rate * 0.0;
+        // the height enters through a softening that follows it
+        const bool massless = r.m[0].mass == 0.0 && r.m[1].mass == 0.0;
+        if (!r.k.constant_softening && !massless)
+            h = div_rn(sqrt_rn(T), root_w2(r.m, xc, yc));  // cbdgam_2d.c:75-106
     }
-    const double T = p[3] / p[0];
-    const bool massless = ms[0].mass == 0.0 && ms[1].mass == 0.0;
-    const double h = massless ? 1.0 : sqrt(T) / root_w2(ms, xc, yc);  // cbdgam_2d.c:75-106
-    mass_source(ms[which - 1], xc, yc, 1.0, p, T, h, r.k.constant_softening, r.k.gm1, r.k.inv_gm1, rate);
+    mass_source(m, xc, yc, 1.0, p, T, h, r.k.constant_softening, r.k.gm1, r.k.inv_gm1, rate);
 }
 
 __device__ __forceinline__ void diag_value(const RedArgs &r, const Diag &d, double x, double y, const double *p,
                                            double *re, double *im)
 {
-    const double rr = sqrt(x * x + y * y);
+    const bool polar = d.quantity == CBD_Q_SIGMA_M1 || d.quantity == CBD_Q_ECCENTRICITY_VECTOR;
+    const double rr = polar || d.has_cut ? sqrt(x * x + y * y) : 0.0;
     const double cut = d.has_cut ? (double)((d.r0 < rr) * (rr < d.r1)) : 1.0;
     *im = 0.0;
     if (d.quantity == CBD_Q_SIGMA_M1) {
@@ -524,10 +547,12 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs r, const do
     for (int q = 0; q < RED_VALUES; ++q)
         v[q] = 0.0;
     const long n = (long)k.ni * k.nj;
-    for (long z = blockIdx.x * (long)RED_THREADS + threadIdx.x; z < n; z += (long)gridDim.x * RED_THREADS) {
-        const int i = (int)(z / k.nj), j = (int)(z % k.nj);
+    const long step = (long)gridDim.x * RED_THREADS, z0 = blockIdx.x * (long)RED_THREADS + threadIdx.x;
+    cbd::ZoneWalk w(z0, step, k.nj);
+    for (long z = z0; z < n; z += step, w.next()) {
+        const int i = w.i, j = w.j;
         const double *p = prim + at(i, j, k.nj);
-        v[0] = max_nan(v[0], max_wavespeed(p, cs2_of(k.gamma, p)));
+        v[0] = max_nan(v[0], max_wavespeed(p, div_rn(p[3], p[0]) * k.gamma));
         const double x = k.xl + (i + 0.5) * k.dx, y = k.yl + (j + 0.5) * k.dy;
         for (int d = 0; d < r.nd; ++d) {
             double re, im;
@@ -551,32 +576,25 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs r, const do
         partials[(size_t)blockIdx.x * RED_VALUES + threadIdx.x] = sm[threadIdx.x][0];
 }
 
-// the blocks' partials to the result: serial in block order, which fixes the sums
-constexpr int FINISH_THREADS = 256, FINISH_CHUNK = 592;
-
-__global__ void __launch_bounds__(FINISH_THREADS) finish_kernel(const double *partials, int nblocks, double *result)
+// The blocks' partials to the result, a warp per value: lane l takes the blocks
+// l, l + 32, ... in order, then a fixed shuffle tree (one thread per value over
+// all blocks took 13 us, most of it the chain of comparisons and additions).
+__global__ void __launch_bounds__(32 * RED_VALUES) finish_kernel(const double *partials, int nblocks, double *result)
 {
-    // the partials through shared memory (loads of a chunk in flight together),
-    // then one thread per value adds them in block order
-    __shared__ double part[FINISH_CHUNK * RED_VALUES];
     cbd::chain_begin();
-    const int q = threadIdx.x;
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double s = 0.0;
-    for (int b0 = 0; b0 < nblocks; b0 += FINISH_CHUNK) {
-        const int n = nblocks - b0 < FINISH_CHUNK ? nblocks - b0 : FINISH_CHUNK;
-        for (int w = q; w < n * RED_VALUES; w += FINISH_THREADS)
-            part[w] = partials[(size_t)b0 * RED_VALUES + w];
-        __syncthreads();
-        if (q < RED_VALUES) {
-#pragma unroll 8
-            for (int b = 0; b < n; ++b) {
-                const double x = part[b * RED_VALUES + q];
-                s = q == 0 ? max_nan(s, x) : s + x;
-            }
-        }
-        __syncthreads();
+#pragma unroll 4
+    for (int b = lane; b < nblocks; b += 32) {
+        const double x = partials[(size_t)b * RED_VALUES + q];
+        s = q == 0 ? max_nan(s, x) : s + x;
     }
-    if (q < RED_VALUES)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_down_sync(0xffffffffu, s, o);
+        s = q == 0 ? max_nan(s, x) : s + x;
+    }
+    if (lane == 0)
         result[q] = s;
 }
 
@@ -1007,7 +1025,7 @@ int cbdgam_b200_reduce(const cbdgam_grid_t *grid, const cbd_mass_t *masses, cons
     const cudaError_t e = cbd::launch_chained(reduce_kernel, RED_BLOCKS, RED_THREADS, 0, s, r, primitive, scratch);
     if (e != cudaSuccess)
         return status_of(e);
-    return status_of(cbd::launch_chained(finish_kernel, 1, FINISH_THREADS, 0, s, scratch, RED_BLOCKS, result));
+    return status_of(cbd::launch_chained(finish_kernel, 1, 32 * RED_VALUES, 0, s, scratch, RED_BLOCKS, result));
 }
 
 }  // extern "C"
