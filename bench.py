@@ -36,15 +36,16 @@ BYTES_PER_ZONE_UPDATE = 120.0  # RK2 x FP64 x 3 fields: 48 B stage 1 + 72 B stag
 # the face cache, the stage-2 launch writing it and the stage-2 epilogue
 # kernel, halved per stage); scaled by the zone count. It is above the
 # algorithmic 60 B because of the cache's 48 B per zone and step and the
-# epilogue's 24 B read-back.
-NCU_TRAFFIC_PER_ZONE_LAUNCH = (316.53e6 + 62.18e6 + 220.12e6 + 249.12e6 + 100.89e6 + 3.63e6) / 2 / 2048 ** 2
+# epilogue's read-back of the state (24 B) and the gravity factors (16 B).
+NCU_TRAFFIC_PER_ZONE_LAUNCH = (315.76e6 + 59.59e6 + 218.99e6 + 248.55e6 + 168.02e6 + 3.47e6) / 2 / 2048 ** 2
 # FP64 thread-instructions (DADD + DMUL + DFMA) per zone and stage, from the
 # same three launches (ncu, the sum of
 # smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma}_pred_on.sum over zones;
 # 2048^2 runs 19-row segments, 4096^2 37-row ones, which recompute fewer
 # rows at segment tops: at 4096^2 this slightly overstates the count)
-FP64_INST_PER_ZONE_LAUNCH = (318.2 + 509.8 + 114.8) / 2
-GAM_FP64_INST_PER_ZONE_LAUNCH = (1224.8 + 1249.8) / 2
+FP64_INST_PER_ZONE_LAUNCH = (296.4 + 451.7 + 53.3) / 2
+# the gamma-law stage at 2048^2 without a face cache role, which is how its kernel is timed below
+GAM_FP64_INST_PER_ZONE_LAUNCH = 930.8
 DIAGNOSTICS = [dict(quantity="time"), dict(quantity="mdot", which_mass=1, accretion=True),
                dict(quantity="mdot", which_mass=2, accretion=True),
                dict(quantity="torque", which_mass="both", gravity=True)]
@@ -507,8 +508,8 @@ def run_ours(args, rank, world):
                 "frac": round(achieved / peak, 4), "traffic": round(NCU_TRAFFIC_PER_ZONE_LAUNCH * zones),
                 "traffic_source": "ncu at 2048^2 scaled by zones",
                 "traffic_note": "above the algorithmic bytes by design: the face cache writes and reads 48 B per "
-                                "zone and step to save FP64 work, and the epilogue reads the new state back "
-                                "(24 B per zone and step); HBM is about 85 % idle",
+                                "zone and step to save FP64 work, and the epilogue reads the new state and the "
+                                "gravity factors back (40 B per zone and step); HBM is about 60 % idle",
                 "peak_source": peak_kind,
                 "kernel": "one RK stage: stage_kernel (mean of the stage-1 reader and the stage-2 writer) with the "
                           "stage-2 epilogue kernel", "kernel_ms": round(kernel_s * 1e3, 4),

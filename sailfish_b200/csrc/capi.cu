@@ -135,14 +135,14 @@ int small_grid_rows(int ni, int strips, int bj, int slots)
 // strips, `slots` CTAs of bj threads resident at a time.
 //
 // Beyond the small grids the CTAs should fill whole waves of the resident
-// slots: a last, partial wave leaves SMs idle at the end of the launch (4096^2
-// at 256 columns: 37 rows, 4.0 waves, 2.127 ms per step; 36 rows, 4.11
-// waves, 2.239 ms; 32 rows, 4.61 waves, 2.150 ms). Each CTA also
-// recomputes about two rows' worth of slopes and faces at its
-// segment's top, and a single wave starts every CTA at once
-// (2048^2: 19 rows in 1.95 waves 0.607 ms, 38 rows in 0.97 waves
-// 0.628 ms; 1024^2 at 128 columns: 10 rows in 0.93 waves 0.212 ms,
-// 5 rows in 1.85 waves 0.219 ms). Score of r rows in W waves:
+// slots: a last, partial wave leaves SMs idle at the end of the launch. Each
+// CTA also recomputes about two rows' worth of slopes and faces at its
+// segment's top, and a single wave starts every CTA at once. Measured at 256
+// columns, us per step by rows (the rule's choice first): 4096^2 37 (4.0 waves)
+// 1612, 32 1621, 25 1626, 38 1640, 36 (4.1) 1669; 2048^2 19 (1.95) 463, 37
+// 467, 13 473, 38 478, 20 479, 18 (2.05) 504; 1511^2 21 (0.97) 286, 11 293, 14
+// 305, 10 311; 1200^2 14 (0.97) 196, 7 200, 15 209, 11 231; 1024^2 10 (0.93)
+// 145, 14 146, 5 150, 9 171. Score of r rows in W waves:
 // (W / ceil(W)) (r / (r + 2)), times 0.95 below 1.5 waves.
 int cbd::segment_rows(int ni, int strips, int bj, int slots)
 {

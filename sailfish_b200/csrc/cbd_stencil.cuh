@@ -13,9 +13,10 @@
 //    operations run on the same operands.
 //  * Boundary conditions are fused: the writer of an edge zone also writes its
 //    zero-gradient guard zones, so the next stage reads valid guards.
-//  * The final stage can fold in the next step's CFL wavespeed and up to
-//    CBD_MAX_FUSED diagnostic sums, reduced deterministically (fixed-order warp
-//    and block trees, then a last-CTA pass over per-CTA partials).
+//  * The final stage is followed by a launch over the same tiles for the next
+//    step's CFL wavespeed and up to CBD_MAX_FUSED diagnostic sums, reduced
+//    deterministically (fixed-order warp and block trees, then a last-CTA pass
+//    over per-CTA partials).
 //
 // PREC selects the arithmetic (CBD_PRECISION_*). EXACT and FMA run identical
 // source (the EXACT translation unit is compiled with -fmad=false) and return
@@ -657,7 +658,7 @@ struct StageArgs {
 //  * ROLE_WRITER (RK2's second stage, RK3's second): computes the values in
 //    its stencil as usual and, when its masses equal its record's
 //    end-of-step masses, also stores them with a key of everything they
-//    depend on (written by one thread).
+//    depend on (by the first CTA, a word per thread).
 //  * ROLE_READER (a step's first stage): a fill kernel runs first; when the
 //    key does not match the stage's masses (a solver's first step, a reset,
 //    the rare time mismatch) it computes every value for them. The stage
