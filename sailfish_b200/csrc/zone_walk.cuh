@@ -14,9 +14,14 @@ struct ZoneWalk {
 
     __device__ __forceinline__ ZoneWalk(long z0, long step, int nj) : nj_(nj)
     {
-        i = (int)(z0 / nj);
+        if ((unsigned long)(z0 | step) >> 32) {
+            i = (int)(z0 / nj);
+            di_ = (int)(step / nj);
+        } else {
+            i = (int)((unsigned)z0 / (unsigned)nj);
+            di_ = (int)((unsigned)step / (unsigned)nj);
+        }
         j = (int)(z0 - (long)i * nj);
-        di_ = (int)(step / nj);
         dj_ = (int)(step - (long)di_ * nj);
     }
     __device__ __forceinline__ void next()

@@ -23,7 +23,8 @@ from sailfish_b200.mesh import PlanarCartesian2DMesh  # noqa: E402
 from sailfish_b200.setups import CircumbinaryDisk  # noqa: E402
 
 
-@pytest.mark.parametrize("shape", [(1, 1), (2, 5), (1, 1300001), (650001, 2), (2000, 701), (1001, 606)])
+@pytest.mark.parametrize("shape", [(1, 1), (2, 5), (33, 31), (40, 32), (1, 1300001), (650001, 2), (2000, 701), (1001, 606),
+                                   (2047, 2051)])
 def test_isothermal_zone_kernels(shape):
     ni, nj = shape
     padded = (ni + 4, nj + 4, 3)
