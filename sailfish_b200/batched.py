@@ -40,11 +40,48 @@ class Disk(NamedTuple):
     solution: Optional[np.ndarray] = None
 
 
-def default_tile(ni, nj):
-    """Tile shape (strip_width, rows) used when no tuned shape is known."""
-    width = 128 if nj > 96 else 64
-    rows = 32 if ni >= 512 else 16
-    return width, rows
+# CTAs of the batched stage kernel resident at a time: 6 on each of 148 SMs
+_SMS, _SLOTS = 148, 148 * 6
+
+
+def default_tiles(sizes):
+    """
+    {(ni, nj): (strip_width, rows)}, the tile shapes of a batch of disks of
+    `sizes` where no tuned ones are known.
+
+    A batch whose tiles of at most 12 rows fit one wave of the resident CTAs
+    takes as long as its fullest SM's march: r rows and a lead-in of about two,
+    at a time per row that grows with the CTAs c there. (r + 2) (3 + 1.25 c)
+    ranks the measured steps (us, rows 1 / 2 / 3 / 4 / 6 / 8 / 16): 3 disks of
+    128^2 to 256^2 68 / 53 / 57 / 60 / 73 / 80 / 128, 4 to 512^2 95 / 85 / 72 /
+    73 / 82 / 90 / 131, 6 to 512^2 163 / 124 / 114 / 118 / 106 / 112 / 146.
+    Larger batches run in waves, largest disks first: tall tiles recompute
+    little at their tops, short ones of the smallest disks fill the end (us,
+    16 rows everywhere / 16 and 32 / 8 and 16 / 8 and 32, from 512^2 on): 12
+    disks to 1024^2 361 / 464 / 360 / 468, 18 disks 577 / 594 / 560 / 594, 24
+    disks 783 / 773 / 777 / 752, 35 disks 1240 / 1215 / 1218 / 1206.
+    """
+    strips = {s: (128 if s[1] > 96 else 64) for s in sizes}
+
+    def tiles(rows):
+        return sum(-(-nj // strips[ni, nj]) * -(-ni // rows) for ni, nj in sizes)
+
+    best = None
+    for rows in range(1, 13):
+        n = tiles(rows)
+        if n <= _SLOTS:
+            cost = (rows + 2.0) * (3.0 + 1.25 * -(-n // _SMS))
+            if best is None or cost < best[0]:
+                best = cost, rows
+    if best is not None:
+        return {s: (strips[s], best[1]) for s in strips}
+    work = tiles(1)  # rows of strips
+    tall, end = (32, 14 * _SLOTS) if work >= 1.4 * 32 * _SLOTS else (16, 9 * _SLOTS)
+    out, short = {}, 0
+    for s in sorted(strips, key=lambda s: s[0] * s[1]):
+        short += sum(-(-t[1] // strips[t]) * t[0] for t in sizes if t == s)
+        out[s] = strips[s], (8 if short <= end else tall)
+    return out
 
 
 class BatchedSolver:
@@ -52,7 +89,7 @@ class BatchedSolver:
     Advance a list of `Disk`s together. `diagnostics` (a list of dicts or
     Diagnostic, at most four besides "time") are reduced for every disk every
     step. `tiles` maps (ni, nj) to (strip_width, rows); missing sizes use
-    `default_tile` unless `autotune` is set, in which case they are measured
+    `default_tiles` unless `autotune` is set, in which case they are measured
     once and cached.
     """
 
@@ -107,7 +144,7 @@ class BatchedSolver:
 
             tiles = dict(tiles or {})
             tiles.update(tuned_tiles(sorted(set(sizes)), precision))
-        tiles = dict(tiles or {})
+        tiles = {**default_tiles(sizes), **(tiles or {})}
         self.tiles = {}
         rec_bytes = int(lib.cbdiso_b200_batch_disk_bytes())
         records = bytearray(rec_bytes * n)
@@ -122,7 +159,7 @@ class BatchedSolver:
         for slot, i in enumerate(self.order):
             s = self.solvers[i]
             ni, nj = s.mesh.shape
-            width, rows = tiles.get((ni, nj), default_tile(ni, nj))
+            width, rows = tiles[ni, nj]
             self.tiles[(ni, nj)] = (width, rows)
             ep = s._epilogue(s.time, True, self._device_diags)
             if lib.cbdiso_b200_epilogue_rates_only(ctypes.byref(ep)) != 1:
