@@ -579,6 +579,15 @@ int cbdgam_b200_advance_stage_cached(const cbdgam_grid_t *grid, const cbdgam_sta
                                      const double *primitive_rd, const double *primitive_n, double *primitive_wr,
                                      double *wavespeed_max, double *face_cache, int role, void *stream);
 
+/* A step's first stage (a = 0): cbdgam_b200_advance_stage_cached without
+ * primitive_n and wavespeed_max (face_cache may be null with role 0), which
+ * also zeroes *wavespeed_clear (device, not null), the maximum that the
+ * step's later stage maxes into: a step needs no launch of its own for that,
+ * and a captured one no state from outside it. */
+int cbdgam_b200_advance_first_stage(const cbdgam_grid_t *grid, const cbdgam_stage_t *stage,
+                                    const double *primitive_rd, double *primitive_wr, double *wavespeed_clear,
+                                    double *face_cache, int role, void *stream);
+
 /* Writes the zero-gradient guard zones of a state from its edge zones
  * (cbdgam_2d.py:491-520 on one patch). */
 int cbdgam_b200_fill_guards(const cbdgam_grid_t *grid, double *primitive, void *stream);

@@ -193,11 +193,7 @@ class Solver(SolverBase):
             self._fcache[:32].zero_()
         # the wavespeed maximum of the current state (slot 0; the multi-GPU
         # solver all-reduces it in place) and, apart, the diagnostic sums
-        # of either of two blocks in turn: a step's second stage needs its slot
-        # zeroed, and the one it will use is cleared a step ahead, while nobody
-        # waits for the launches
-        self._results = [torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, **f64) for _ in range(2)]
-        self._result = self._results[0]
+        self._result = torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, **f64)
         self._sums = torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, **f64)
         self._result_host = torch.zeros(1 + 2 * _capi.GAM_MAX_DIAG, dtype=torch.float64).pin_memory()
         self._result_np = self._result_host.numpy()
@@ -228,16 +224,21 @@ class Solver(SolverBase):
         st.a, st.dt = a, dt
         return st
 
-    def _launch(self, st, rd, pn, wr, ws, role, stream):
+    def _launch(self, st, rd, pn, wr, role, stream):
         """One product stage; `role` (1 writer, 2 reader) is used when the
-        solver keeps a face cache."""
-        lib, g = self._lib, self._grid
-        args = (ctypes.byref(g), ctypes.byref(st), self._ptr(rd), self._ptr(pn) if pn is not None else None,
-                self._ptr(wr), self._ptr(ws) if ws is not None else None)
-        if self._fcache is not None and role:
-            status = lib.cbdgam_b200_advance_stage_cached(*args, self._ptr(self._fcache), role, stream)
+        solver keeps a face cache. The first (no `pn`) zeroes the wavespeed
+        maximum on the device, the second maxes into it: a step carries all it
+        needs, whether it runs now or is captured and replayed."""
+        lib = self._lib
+        cache = self._ptr(self._fcache) if self._fcache is not None and role else None
+        args = ctypes.byref(self._grid), ctypes.byref(st), self._ptr(rd)
+        wr, ws = self._ptr(wr), self._ptr(self._result)
+        if pn is None:
+            status = lib.cbdgam_b200_advance_first_stage(*args, wr, ws, cache, role if cache else 0, stream)
+        elif cache:
+            status = lib.cbdgam_b200_advance_stage_cached(*args, self._ptr(pn), wr, ws, cache, role, stream)
         else:
-            status = lib.cbdgam_b200_advance_stage(*args, stream)
+            status = lib.cbdgam_b200_advance_stage(*args, self._ptr(pn), wr, ws, stream)
         self._check(status, "advance_stage")
 
     @staticmethod
@@ -329,32 +330,24 @@ class Solver(SolverBase):
         """One RK2 step (cbdgam_2d.py:473-489): two stage kernels, masses at
         each stage's start time, the stage times as the reference updates
         them."""
-        import torch
-
         dt = float(dt)
         if not math.isfinite(dt):
             raise _capi.CbdError(_capi.NONFINITE, "advance: time step")
-        lib = self._lib
         stream = self._stream()
         t0 = self._time
         t1 = t0 * 0.0 + (t0 + dt) * (1.0 - 0.0)
         t2 = t0 * 0.5 + (t1 + dt) * (1.0 - 0.5)
         a_buf, b_buf = self._buf
         s1 = self._stage(t0, 0.0, dt)
-        self._launch(s1, a_buf, None, b_buf, None, 2, stream)
+        self._ws_valid = False
+        self._launch(s1, a_buf, None, b_buf, 2, stream)
         if self._stage_hook is not None:
             self._stage_hook(0, b_buf)
         # the second stage's orbit is solved while the first stage runs; it
         # fills the face cache when its masses are the step's end masses
         s2 = self._stage(t1, 0.5, dt)
         writer = self._same_masses(s2, self._stage(t2, 0.5, dt))
-        old, new = self._result, self._results[1 if self._result is self._results[0] else 0]
-        if torch.cuda.is_current_stream_capturing():
-            # a captured step may be replayed alone: it clears its own slot
-            self._check(lib.cbdiso_b200_clear(new.data_ptr(), 8, stream), "clear")
-        self._launch(s2, b_buf, a_buf, a_buf, new, 1 if writer else 0, stream)
-        self._result = new
-        self._check(lib.cbdiso_b200_clear(old.data_ptr(), 8, stream), "clear")
+        self._launch(s2, b_buf, a_buf, a_buf, 1 if writer else 0, stream)
         if self._stage_hook is not None:
             self._stage_hook(1, a_buf)
         self._time = t2

@@ -59,6 +59,7 @@ struct Stage {
     int massless;  // both masses have zero mass: every scale height is 1
     int write_guards;
     int un_from_primitive;  // u_n = cons(primitive_n) in-kernel (else: a conserved array)
+    double *ws_clear;  // zeroed by the stage (or null): the maximum that a later stage of the step maxes into
 };
 
 // Powers and the exponential are correctly rounded (cr_math.cuh): in a
@@ -926,9 +927,16 @@ int cbdgam_2d_point_mass_source_term(int ni, int nj, double xl, double xr, doubl
 
 namespace {
 
+bool cache_ok(const double *face_cache, int role)
+{
+    // the zone pairs are moved as 16-byte vectors
+    return face_cache && (reinterpret_cast<uintptr_t>(face_cache) & 15) == 0 && role >= ROLE_NONE &&
+           role <= ROLE_READER;
+}
+
 int advance_stage(const cbdgam_grid_t *grid, const cbdgam_stage_t *stage, const double *primitive_rd,
                   const double *primitive_n, double *primitive_wr, double *wavespeed_max, double *face_cache,
-                  int role, void *stream)
+                  int role, void *stream, double *wavespeed_clear = nullptr)
 {
     if (!grid_ok(grid) || !stage || !primitive_rd || !primitive_wr || primitive_wr == primitive_rd)
         return CBD_ERR_ARGUMENT;
@@ -948,6 +956,7 @@ int advance_stage(const cbdgam_grid_t *grid, const cbdgam_stage_t *stage, const 
     st.dt = stage->dt;
     st.write_guards = 1;
     st.un_from_primitive = 1;
+    st.ws_clear = wavespeed_clear;
     return launch_stage(consts_of(grid), st, primitive_rd, primitive_n, nullptr, primitive_wr, wavespeed_max,
                         static_cast<cudaStream_t>(stream), face_cache, role);
 }
@@ -974,12 +983,20 @@ int cbdgam_b200_advance_stage_cached(const cbdgam_grid_t *grid, const cbdgam_sta
                                      const double *primitive_rd, const double *primitive_n, double *primitive_wr,
                                      double *wavespeed_max, double *face_cache, int role, void *stream)
 {
-    // the zone pairs are moved as 16-byte vectors
-    if (!face_cache || (reinterpret_cast<uintptr_t>(face_cache) & 15) != 0 || role < ROLE_NONE ||
-        role > ROLE_READER)
+    if (!cache_ok(face_cache, role))
         return CBD_ERR_ARGUMENT;
     return advance_stage(grid, stage, primitive_rd, primitive_n, primitive_wr, wavespeed_max, face_cache, role,
                          stream);
+}
+
+int cbdgam_b200_advance_first_stage(const cbdgam_grid_t *grid, const cbdgam_stage_t *stage,
+                                    const double *primitive_rd, double *primitive_wr, double *wavespeed_clear,
+                                    double *face_cache, int role, void *stream)
+{
+    if (!wavespeed_clear || (role != ROLE_NONE && !cache_ok(face_cache, role)))
+        return CBD_ERR_ARGUMENT;
+    return advance_stage(grid, stage, primitive_rd, nullptr, primitive_wr, nullptr, face_cache, role, stream,
+                         wavespeed_clear);
 }
 
 int cbdgam_b200_fill_guards(const cbdgam_grid_t *grid, double *primitive, void *stream)

@@ -94,6 +94,8 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
     MarchSmem<BJ> &sm = *reinterpret_cast<MarchSmem<BJ> *>(smem_raw);
     cbd::chain_begin();
     const int t = threadIdx.x;
+    if (st.ws_clear && blockIdx.x == 0 && blockIdx.y == 0 && t == 0)
+        *st.ws_clear = 0.0;
     const int ni = k.ni, nj = k.nj;
     const int c0 = blockIdx.x * BJ, r0 = blockIdx.y * rows;
     const int W = min(BJ, nj - c0), r1 = min(r0 + rows, ni);

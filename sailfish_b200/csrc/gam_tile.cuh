@@ -263,6 +263,8 @@ __global__ void __launch_bounds__(NT, TILE_MIN_BLOCKS) tile_kernel(Consts k, Sta
     const int i0 = blockIdx.y * TI, j0 = blockIdx.x * TJ;
     const int ni = k.ni, nj = k.nj;
     const int tid = threadIdx.y * TJ + threadIdx.x;
+    if (st.ws_clear && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0)
+        *st.ws_clear = 0.0;
     for (int s = tid; s < HI * HJ; s += NT) {
         const int ii = i0 - NG + s / HJ, jj = j0 - NG + s % HJ;
         if (ii <= ni + 1 && jj <= nj + 1) {
