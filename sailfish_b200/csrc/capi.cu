@@ -588,15 +588,22 @@ int cbdiso_b200_read(void *dst, const void *src, size_t bytes, void *stream)
     if (!dst || !src)
         return CBD_ERR_ARGUMENT;
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-    return status_of(e == cudaSuccess ? cudaStreamSynchronize(s) : e);
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess)
+        cudaGetLastError();  // not left for a later call to find
+    return status_of(e);
 }
 
 int cbdiso_b200_clear(void *dst, size_t bytes, void *stream)
 {
     if (!dst)
         return CBD_ERR_ARGUMENT;
-    return status_of(cudaMemsetAsync(dst, 0, bytes, static_cast<cudaStream_t>(stream)));
+    const cudaError_t e = cudaMemsetAsync(dst, 0, bytes, static_cast<cudaStream_t>(stream));
+    if (e != cudaSuccess)
+        cudaGetLastError();
+    return status_of(e);
 }
 
 int cbdiso_b200_eval_primitives(long n, const double *a, const double *b, double *out, void *stream)

@@ -27,6 +27,8 @@ __device__ __forceinline__ void chain_begin()
 
 __device__ __forceinline__ void chain_end() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
+// A launch that fails leaves no error behind for a later call to find (the
+// other entry points ask for the last error after their launches).
 template <class... P, class... A>
 cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args)
 {
@@ -40,7 +42,10 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (e != cudaSuccess)
+        cudaGetLastError();
+    return e;
 }
 
 }  // namespace cbd
