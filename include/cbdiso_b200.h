@@ -588,6 +588,11 @@ int cbdgam_b200_advance_first_stage(const cbdgam_grid_t *grid, const cbdgam_stag
                                     const double *primitive_rd, double *primitive_wr, double *wavespeed_clear,
                                     double *face_cache, int role, void *stream);
 
+/* Columns of a CTA of the stage kernel that the grid takes (host only; the
+ * results do not depend on it): 64 or 128, a strip of the row march, or 32, a
+ * tile of 16 rows. 0 for an invalid grid. */
+int cbdgam_b200_stage_columns(const cbdgam_grid_t *grid);
+
 /* Writes the zero-gradient guard zones of a state from its edge zones
  * (cbdgam_2d.py:491-520 on one patch). */
 int cbdgam_b200_fill_guards(const cbdgam_grid_t *grid, double *primitive, void *stream);

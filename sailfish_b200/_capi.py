@@ -213,6 +213,7 @@ def _declare(lib):
         "cbdgam_b200_advance_stage": [POINTER(GamGrid), POINTER(GamStage), V, V, V, V, V],
         "cbdgam_b200_advance_stage_cached": [POINTER(GamGrid), POINTER(GamStage), V, V, V, V, V, I, V],
         "cbdgam_b200_advance_first_stage": [POINTER(GamGrid), POINTER(GamStage), V, V, V, V, I, V],
+        "cbdgam_b200_stage_columns": [POINTER(GamGrid)],
         "cbdgam_b200_fill_guards": [POINTER(GamGrid), V, V],
         "cbdgam_b200_reduce": [POINTER(GamGrid), POINTER(Mass), POINTER(Diag), c_int, V, V, V, V],
         "cbdgam_b200_eval_powers": [ctypes.c_long, V, V, V],
@@ -279,7 +280,7 @@ def exported_symbols():
         "cbdgam_2d_advance_rk", "cbdgam_2d_wavespeed", "cbdgam_2d_primitive_to_conserved",
         "cbdgam_2d_point_mass_source_term", "cbdgam_b200_set_plm_theta", "cbdgam_b200_advance_stage",
         "cbdgam_b200_face_cache_bytes", "cbdgam_b200_advance_stage_cached", "cbdgam_b200_advance_first_stage",
-        "cbdgam_b200_fill_guards", "cbdgam_b200_scratch_bytes", "cbdgam_b200_reduce", "cbdgam_b200_abi_sizes",
+        "cbdgam_b200_stage_columns", "cbdgam_b200_fill_guards", "cbdgam_b200_scratch_bytes", "cbdgam_b200_reduce", "cbdgam_b200_abi_sizes",
         "cbdgam_b200_eval_powers", "cbdiso_b200_fp64_probe", "cbdiso_b200_fp64_probe_fmas",
         "cbdgam_b200_disk_primitive",
     ]

@@ -736,12 +736,19 @@ int launch_tiles(const Consts &k, const Stage &st, const double *prd, const doub
 
 // The march where its CTAs hold one row each and all fit at once (the latency
 // of one zone's update is what counts there), and on large grids, where its
-// segments are long, unless a last strip of few columns takes up its slots; the
-// tiles between. Measured, us per step, tiles / march: 64^2 30 / 20, 130^2 29 /
-// 23, 200^2 30 / 26, 256^2 30 / 32, 384^2 38 / 50, 512^2 66 / 69, 704^2 111 /
-// 126, 900^2 175 / 188, 1000^2 227 / 216, 1280^2 358 / 323, 2048^2 870 / 760
-// (with cooling 238 / 228, 377 / 345, 920 / 818); 1153^2, with a tenth strip of
-// one column, 294 / 300 and with cooling 310 / 318.
+// segments are long; the tiles between. Measured, us per step, tiles / march:
+// 64^2 30 / 20, 130^2 29 / 23, 200^2 30 / 26, 256^2 30 / 32, 384^2 38 / 50, 512^2
+// 66 / 69, 704^2 111 / 126, 900^2 175 / 188, 1000^2 227 / 216, 1280^2 358 / 323,
+// 2048^2 870 / 760 (with cooling 238 / 228, 377 / 345, 920 / 818).
+//
+// A last strip of few columns takes up the march's slots like a full one, so on
+// a large grid its strips may hold at most 8 % more columns than the tiles'
+// 32-column ones: 13000 x 130 428 / 591 (strips of 256 against 160 columns),
+// 13000 x 200 600 / 654, 8000 x 260 478 / 555, 8000 x 300 528 / 559, 4096 x 385
+// 358 / 445, 1153^2 294 / 300, 1700 x 1025 373 / 377 (1.09); 1281^2 356 / 342
+// (1.07), 1024 x 1800 396 / 399 (1.05), 2600 x 640 346 / 348, 13000 x 256 681 /
+// 649, 26000 x 100 675 / 651, 300 x 8000 517 / 470. Its 64-column strips serve
+// small grids only: 26000 x 60 350 / 367, 26000 x 96 519 / 704.
 // Strips of 128 columns at 3 CTAs per SM, narrow grids in 64 columns.
 constexpr int MARCH_CTAS = 3;
 
@@ -750,18 +757,25 @@ bool march_suits(int ni, int nj)
     const long strips = (nj + 127) / 128, zones = (long)ni * nj;
     if (strips * ni <= 148 * MARCH_CTAS * (nj <= 96 ? 2 : 1))
         return true;
-    return zones >= 1280L * 1280 || (zones >= 960L * 960 && strips * 128 <= 1.08 * nj);
+    const long tile_columns = (nj + TJ - 1) / TJ * TJ;
+    return zones >= 960L * 960 && nj > 96 && strips * 128 <= 1.08 * tile_columns;
 }
+
+// columns of a CTA of the stage kernel
+int stage_columns(int ni, int nj) { return !march_suits(ni, nj) ? TJ : (nj <= 96 ? 64 : 128); }
 
 template <int ROLE>
 int launch_role(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
                 double *pwr, double *ws_max, double *fc, cudaStream_t s)
 {
-    if (!march_suits(k.ni, k.nj))
+    switch (stage_columns(k.ni, k.nj)) {
+    case TJ:
         return launch_tiles<ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
-    if (k.nj <= 96)
+    case 64:
         return launch_march<64, 2 * MARCH_CTAS, ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
-    return launch_march<128, MARCH_CTAS, ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
+    default:
+        return launch_march<128, MARCH_CTAS, ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
+    }
 }
 
 int launch_stage(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
@@ -997,6 +1011,11 @@ int cbdgam_b200_advance_first_stage(const cbdgam_grid_t *grid, const cbdgam_stag
         return CBD_ERR_ARGUMENT;
     return advance_stage(grid, stage, primitive_rd, nullptr, primitive_wr, nullptr, face_cache, role, stream,
                          wavespeed_clear);
+}
+
+int cbdgam_b200_stage_columns(const cbdgam_grid_t *grid)
+{
+    return grid_ok(grid) ? stage_columns(grid->ni, grid->nj) : 0;
 }
 
 int cbdgam_b200_fill_guards(const cbdgam_grid_t *grid, double *primitive, void *stream)
