@@ -365,7 +365,7 @@ __device__ __forceinline__ void cons_to_prim(const double *u, double *p, const C
 // max |v +- cs| over both directions, cbdiso_2d.c:340-350
 __device__ __forceinline__ double max_wavespeed(const double *p, double cs2)
 {
-    const double cs = crm::sqrt_rn(cs2);
+    const double cs = crm::sqrt_any(cs2);
     const double ax = greater(fabs(p[1] - cs), fabs(p[1] + cs));
     const double ay = greater(fabs(p[2] - cs), fabs(p[2] + cs));
     return greater(ax, ay);

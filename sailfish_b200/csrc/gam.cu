@@ -105,6 +105,40 @@ __device__ __forceinline__ double div_by(double a, double b, double y)
 
 __device__ __forceinline__ double div_rn(double a, double b) { return div_by(a, b, recip_rn(b)); }
 
+// T = p / Sigma, the sound speed sqrt(T gamma) (cbdgam_2d.c:231-236) and sqrt(T)
+struct Thermal {
+    double T, cs, sq;
+};
+
+// for any pressure and density, by CUDA's operators; out of line, where its
+// callers go only for arguments that the straight-line ones do not cover
+__device__ __noinline__ Thermal thermal_any(double pres, double sigma, double gamma)
+{
+    Thermal r;
+    r.T = pres / sigma;
+    r.cs = sqrt(r.T * gamma);
+    r.sq = sqrt(r.T);
+    return r;
+}
+
+__device__ __forceinline__ bool thermal_in_range(double pres, double T)
+{
+    return crm::mid_range(pres) && crm::mid_range(T);
+}
+
+// WIDE: any pressure and density (stage_wide says when a stage needs that)
+template <bool WIDE>
+__device__ __forceinline__ Thermal thermal(double pres, double sigma, double gamma)
+{
+    Thermal r;
+    r.T = div_rn(pres, sigma);
+    r.cs = sqrt_rn(r.T * gamma);
+    r.sq = sqrt_rn(r.T);
+    if (WIDE && !thermal_in_range(pres, r.T))
+        r = thermal_any(pres, sigma, gamma);
+    return r;
+}
+
 // cbdgam_2d.c:238-276
 __device__ __forceinline__ void buffer_source(const Consts &k, const Stage &st, double x, double y, double dt,
                                               double *u)
@@ -137,14 +171,23 @@ __device__ __forceinline__ void prim_to_cons(const V &p, double *u, double gamma
     u[3] = pres / (gamma - 1.0) + 0.5 * rho * (vx * vx + vy * vy);
 }
 
-// cbdgam_2d.c:401-409
+// cbdgam_2d.c:401-409 for a sound speed
 template <class V>
-__device__ __forceinline__ double max_wavespeed(const V &p, double cs2)
+__device__ __forceinline__ double max_wavespeed(const V &p, double cs)
 {
-    const double cs = sqrt_rn(cs2);
     const double ax = greater(fabs(p[1] - cs), fabs(p[1] + cs));
     const double ay = greater(fabs(p[2] - cs), fabs(p[2] + cs));
     return greater(ax, ay);
+}
+
+// the same of a zone with any pressure and density
+__device__ __forceinline__ double zone_wavespeed(const double *p, double gamma)
+{
+    const double T = div_rn(p[3], p[0]);
+    double cs = sqrt_rn(T * gamma);
+    if (!thermal_in_range(p[3], T))
+        cs = thermal_any(p[3], p[0], gamma).cs;
+    return max_wavespeed(p, cs);
 }
 
 // sqrt(w2) of the scale height (cbdgam_2d.c:75-106) at (x, y)
@@ -246,6 +289,18 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
     }
 }
 
+// 2^-298 <= |x| < 2^298, by the exponent field: within 1e-90 to 1e90
+__device__ __forceinline__ bool power_range(double x)
+{
+    return ((unsigned)__double2hiint(x) & 0x7fffffffu) - 0x2d500000u < 0x25400000u;
+}
+
+// cooling's factor for any argument, out of line
+__device__ __noinline__ double cooling_factor(double cooling, double sigma, double eps, double dt)
+{
+    return pow_m13_rn(1.0 + 3.0 * cooling * inv_square_rn(sigma) * cube_rn(eps) * dt);
+}
+
 // cbdgam_2d.c:298-317 with T = p / Sigma given
 template <class V>
 __device__ __forceinline__ void cooling_fast(const Consts &k, double dt, const V &p, double T, double *u)
@@ -254,9 +309,16 @@ __device__ __forceinline__ void cooling_fast(const Consts &k, double dt, const V
     const double eps = div_by(T, k.gm1, k.inv_gm1);
     // without cooling the power's argument is exactly 1 and so is the power
     // (for finite Sigma^-2 eps^3, which the floors keep)
-    double cooled = k.cooling == 0.0
-                        ? eps
-                        : eps * pow_m13_rn(1.0 + 3.0 * k.cooling * inv_square_rn(sigma) * cube_rn(eps) * dt);
+    double cooled = eps;
+    if (k.cooling != 0.0) {
+        const double x = 1.0 + 3.0 * k.cooling * crm::inv_square_in(sigma) * crm::cube_in(eps) * dt;
+        double w = crm::pow_m13_in(x);
+        // outside the powers' safe ranges, 1e-90 to 1e90 in magnitude and 1 to
+        // 1e90, or thereabouts (by the exponent fields)
+        if (!(power_range(sigma) && power_range(eps) && (unsigned)(__double2hiint(x) - 0x3ff00000) < 0x12a00000u))
+            w = cooling_factor(k.cooling, sigma, eps, dt);
+        cooled *= w;
+    }
     const double ek = 0.5 * (p[1] * p[1] + p[2] * p[2]);
     cooled = greater(cooled, div_by(div_by(2.0 * ek, k.gamma, k.inv_gamma), k.gm1, k.inv_gm1) * k.mach_m2);
     u[3] += sigma * (cooled - eps);
@@ -410,7 +472,7 @@ __global__ void wavespeed_kernel(int ni, int nj, double gamma, const double *pri
     for (long z = z0; z < n; z += step, w.next()) {
         const int i = w.i, j = w.j;
         const double *p = prim + at(i, j, nj);
-        ws[(size_t)(i + NG) * (nj + 2 * NG) + (j + NG)] = max_wavespeed(p, cs2_of(gamma, p));
+        ws[(size_t)(i + NG) * (nj + 2 * NG) + (j + NG)] = max_wavespeed(p, sqrt(cs2_of(gamma, p)));
     }
 }
 
@@ -479,7 +541,7 @@ __device__ __forceinline__ void diag_rates(const RedArgs &r, const Diag &d, int 
                                            const double *p, double *rate)
 {
     Mass m = r.m[which - 1];
-    const double T = div_rn(p[3], p[0]);
+    const double T = p[3] / p[0];  // enters through the height alone
     double h = 1.0;
     if (d.accretion) {
         // without masses every height is 1; beyond the sink's reach the rates are
@@ -498,7 +560,7 @@ __device__ __forceinline__ void diag_rates(const RedArgs &r, const Diag &d, int 
         // the height enters through a softening that follows it
         const bool massless = r.m[0].mass == 0.0 && r.m[1].mass == 0.0;
         if (!r.k.constant_softening && !massless)
-            h = div_rn(sqrt_rn(T), root_w2(r.m, xc, yc));  // cbdgam_2d.c:75-106
+            h = sqrt(T) / root_w2(r.m, xc, yc);  // cbdgam_2d.c:75-106
     }
     mass_source(m, xc, yc, 1.0, p, T, h, r.k.constant_softening, r.k.gm1, r.k.inv_gm1, rate);
 }
@@ -553,7 +615,7 @@ __global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs r, const do
     for (long z = z0; z < n; z += step, w.next()) {
         const int i = w.i, j = w.j;
         const double *p = prim + at(i, j, k.nj);
-        v[0] = max_nan(v[0], max_wavespeed(p, div_rn(p[3], p[0]) * k.gamma));
+        v[0] = max_nan(v[0], zone_wavespeed(p, k.gamma));
         const double x = k.xl + (i + 0.5) * k.dx, y = k.yl + (j + 0.5) * k.dy;
         for (int d = 0; d < r.nd; ++d) {
             double re, im;
@@ -701,36 +763,36 @@ int launch_fill(const Consts &k, const Stage &st, double *fc, cudaStream_t s)
     return status_of(cbd::launch_chained(cache_fill_kernel, rows, 128, 0, s, k, st, fc));
 }
 
-template <int BJ, int MINB, int ROLE>
+template <int BJ, int MINB, int ROLE, bool WIDE>
 int launch_march(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
                  double *pwr, double *ws_max, double *fc, cudaStream_t s)
 {
     static bool ready[64] = {};
     const int smem = (int)sizeof(MarchSmem<BJ>);
-    int rc = prepare_kernel(reinterpret_cast<const void *>(stage_kernel<BJ, MINB, ROLE>), smem, ready);
+    int rc = prepare_kernel(reinterpret_cast<const void *>(stage_kernel<BJ, MINB, ROLE, WIDE>), smem, ready);
     if (rc == CBD_OK && ROLE == ROLE_READER)
         rc = launch_fill(k, st, fc, s);
     if (rc != CBD_OK)
         return rc;
     const int strips = (k.nj + BJ - 1) / BJ;
     const int rows = cbd::segment_rows(k.ni, strips, BJ, 148 * MINB);
-    return status_of(cbd::launch_chained(stage_kernel<BJ, MINB, ROLE>, dim3(strips, (k.ni + rows - 1) / rows), BJ, smem,
+    return status_of(cbd::launch_chained(stage_kernel<BJ, MINB, ROLE, WIDE>, dim3(strips, (k.ni + rows - 1) / rows), BJ, smem,
                                          s, k, st, rows, prd, pn, un, pwr,
                                          reinterpret_cast<unsigned long long *>(ws_max), fc));
 }
 
-template <int ROLE>
+template <int ROLE, bool WIDE>
 int launch_tiles(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
                  double *pwr, double *ws_max, double *fc, cudaStream_t s)
 {
     static bool ready[64] = {};
-    int rc = prepare_kernel(reinterpret_cast<const void *>(tile_kernel<ROLE>), (int)sizeof(TileSmem), ready);
+    int rc = prepare_kernel(reinterpret_cast<const void *>(tile_kernel<ROLE, WIDE>), (int)sizeof(TileSmem), ready);
     if (rc == CBD_OK && ROLE == ROLE_READER)
         rc = launch_fill(k, st, fc, s);
     if (rc != CBD_OK)
         return rc;
     const dim3 grid((k.nj + TJ - 1) / TJ, (k.ni + TI - 1) / TI), block(TJ, TI / RPT);
-    return status_of(cbd::launch_chained(tile_kernel<ROLE>, grid, block, sizeof(TileSmem), s, k, st, prd, pn, un, pwr,
+    return status_of(cbd::launch_chained(tile_kernel<ROLE, WIDE>, grid, block, sizeof(TileSmem), s, k, st, prd, pn, un, pwr,
                                          reinterpret_cast<unsigned long long *>(ws_max), fc));
 }
 
@@ -764,18 +826,34 @@ bool march_suits(int ni, int nj)
 // columns of a CTA of the stage kernel
 int stage_columns(int ni, int nj) { return !march_suits(ni, nj) ? TJ : (nj <= 96 ? 64 : 128); }
 
-template <int ROLE>
-int launch_role(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
+template <int ROLE, bool WIDE>
+int launch_form(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
                 double *pwr, double *ws_max, double *fc, cudaStream_t s)
 {
     switch (stage_columns(k.ni, k.nj)) {
     case TJ:
-        return launch_tiles<ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
+        return launch_tiles<ROLE, WIDE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
     case 64:
-        return launch_march<64, 2 * MARCH_CTAS, ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
+        return launch_march<64, 2 * MARCH_CTAS, ROLE, WIDE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
     default:
-        return launch_march<128, MARCH_CTAS, ROLE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
+        return launch_march<128, MARCH_CTAS, ROLE, WIDE>(k, st, prd, pn, un, pwr, ws_max, fc, s);
     }
+}
+
+// Whether a stage may meet temperatures outside the range of the straight-line
+// roots. The test splits the march's longest chain: 2048^2 743 -> 761 us per
+// step, 1153^2 (tiles) 290 -> 291. With a pressure floor above 1e-90 only
+// densities above 1e198, or an initial state below the floor whose sound speed
+// (below 1e-144) moves nothing, could have one; without such a floor a cold gas
+// can.
+bool stage_wide(const Consts &k) { return !(k.p_floor > 1e-90); }
+
+template <int ROLE>
+int launch_role(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,
+                double *pwr, double *ws_max, double *fc, cudaStream_t s)
+{
+    return stage_wide(k) ? launch_form<ROLE, true>(k, st, prd, pn, un, pwr, ws_max, fc, s)
+                         : launch_form<ROLE, false>(k, st, prd, pn, un, pwr, ws_max, fc, s);
 }
 
 int launch_stage(const Consts &k, const Stage &st, const double *prd, const double *pn, const double *un,

@@ -78,14 +78,14 @@ struct MarchSmem {
 // (the reference's conserved_rk array). With ws_max set, the largest
 // wavespeed of the written zones is max-ed into it (non-negative doubles
 // order as their bit patterns do). ROLE (ROLE_*) is what the stage does with
-// the face cache `fc`.
+// the face cache `fc`; WIDE as in thermal.
 //
 // Ring slot of row i: (i - r0 + 2) mod 5. Iteration r reads rows r .. r + 2;
 // row r + 4 is fetched after its barrier into the slot of row r - 1, and each
 // thread has waited for its copies of row r + 3 before the barrier. zone[]
 // of row r + 1 and north[] of row r alternate between two buffers by row
 // parity, so that a warp ahead of the others writes beside what they read.
-template <int BJ, int MINB, int ROLE>
+template <int BJ, int MINB, int ROLE, bool WIDE>
 __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const Stage st, const int rows,
                                                          const double *prd, const double *pn, const double *un_all,
                                                          double *pwr, unsigned long long *ws_max, double *fc)
@@ -143,9 +143,10 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
             v.gx[q] = slope(zl[q], zc[q], zr[q], k.theta);
             gy[q] = slope(a[q], zc[q], b[q], k.theta);
         }
-        v.T = div_rn(zc[3], zc[0]);
-        v.cs = sqrt_rn(v.T * k.gamma);  // cs2 = p / Sigma * gamma (cbdgam_2d.c:231-236)
-        v.sq = sqrt_rn(v.T);
+        const Thermal th = thermal<WIDE>(zc[3], zc[0], k.gamma);
+        v.T = th.T;
+        v.cs = th.cs;
+        v.sq = th.sq;
         // strain (cbdgam_2d.c:278-294): (4/3 gx_vx) / dx - (2/3 gy_vy) / dy, ...
         v.sxx = div_by(4.0 / 3.0 * v.gx[1], k.dx, k.inv_dx) - div_by(2.0 / 3.0 * gy[2], k.dy, k.inv_dy);
         v.sxy = div_by(v.gx[2], k.dx, k.inv_dx) + div_by(gy[1], k.dy, k.inv_dy);
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
                     }
             }
             if (ws_max)
-                ws = max_nan(ws, max_wavespeed(out, div_rn(out[3], out[0]) * k.gamma));
+                ws = max_nan(ws, zone_wavespeed(out, k.gamma));
         }
         // into the buffers this iteration has read; landed by the next barrier
         fetch_own(r + 2);

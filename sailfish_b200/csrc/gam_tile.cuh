@@ -53,7 +53,7 @@ __device__ __forceinline__ void hlle_fast(const Consts &k, const double *pl, con
 
 // Phase 1: the per-zone quantities of zone (i0 - 1 + a, j0 - 1 + b) and the
 // face geometry of the tile.
-template <int ROLE>
+template <int ROLE, bool WIDE>
 __device__ __forceinline__ void tile_phase1(const Consts &k, const Stage &st, TileSmem &sm, int i0, int j0, int tid,
                                              const CacheView &cv)
 {
@@ -110,10 +110,10 @@ __device__ __forceinline__ void tile_phase1(const Consts &k, const Stage &st, Ti
             sm.z[Q_GX + q][a][b] = gx[q];
             sm.z[Q_GY + q][a][b] = gy[q];
         }
-        const double T = div_rn(sm.prim[3][a + 1][b + 1], sm.prim[0][a + 1][b + 1]);
-        sm.z[Q_T][a][b] = T;
-        sm.z[Q_CS][a][b] = sqrt_rn(T * k.gamma);  // sqrt(cs2), cs2 = p / Sigma * gamma (cbdgam_2d.c:231-236)
-        sm.z[Q_SQ][a][b] = sqrt_rn(T);
+        const Thermal th = thermal<WIDE>(sm.prim[3][a + 1][b + 1], sm.prim[0][a + 1][b + 1], k.gamma);
+        sm.z[Q_T][a][b] = th.T;
+        sm.z[Q_CS][a][b] = th.cs;
+        sm.z[Q_SQ][a][b] = th.sq;
         // strain (cbdgam_2d.c:278-294): (4/3 gx_vx) / dx - (2/3 gy_vy) / dy, ...
         sm.z[Q_SXX][a][b] = div_by(4.0 / 3.0 * gx[1], k.dx, k.inv_dx) - div_by(2.0 / 3.0 * gy[2], k.dy, k.inv_dy);
         sm.z[Q_SXY][a][b] = div_by(gx[2], k.dx, k.inv_dx) + div_by(gy[1], k.dy, k.inv_dy);
@@ -248,8 +248,8 @@ __device__ __forceinline__ void tile_phase2(const Consts &k, const Stage &st, co
 // or un_all does (the reference's conserved_rk array). With ws_max set, the
 // largest wavespeed of the written zones is max-ed into it (non-negative
 // doubles order as their bit patterns do).
-// ROLE (ROLE_*) is what the stage does with the face cache `fc`.
-template <int ROLE>
+// ROLE (ROLE_*) is what the stage does with the face cache `fc`; WIDE as in thermal.
+template <int ROLE, bool WIDE>
 __global__ void __launch_bounds__(NT, TILE_MIN_BLOCKS) tile_kernel(Consts k, Stage st,
                                                                           const double *prd,
                                                                           const double *pn,
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(NT, TILE_MIN_BLOCKS) tile_kernel(Consts k, Sta
         if (ROLE == ROLE_WRITER && blockIdx.x == 0 && blockIdx.y == 0 && tid < CACHE_KEY)
             fc[tid] = cache_key_value(k, st.m, tid);
     }
-    tile_phase1<ROLE>(k, st, sm, i0, j0, tid, cv);
+    tile_phase1<ROLE, WIDE>(k, st, sm, i0, j0, tid, cv);
     __syncthreads();
     double ws = 0.0;
 #pragma unroll 1
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(NT, TILE_MIN_BLOCKS) tile_kernel(Consts k, Sta
                     dst[q] = out[q];
             }
         if (ws_max)
-            ws = max_nan(ws, max_wavespeed(out, div_rn(out[3], out[0]) * k.gamma));
+            ws = max_nan(ws, zone_wavespeed(out, k.gamma));
     }
     cbd::chain_end();
     if (ws_max) {  // uniform over the block
