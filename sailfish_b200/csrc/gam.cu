@@ -123,7 +123,7 @@ __device__ __noinline__ Thermal thermal_any(double pres, double sigma, double ga
 
 __device__ __forceinline__ bool thermal_in_range(double pres, double T)
 {
-    return crm::mid_range(pres) && crm::mid_range(T);
+    return crm::mid_range(pres) & crm::mid_range(T);
 }
 
 // WIDE: any pressure and density (stage_wide says when a stage needs that)
@@ -215,9 +215,18 @@ __device__ __forceinline__ void p2c_fast(const Consts &k, const V &p, double *u)
     u[3] = div_by(pres, k.gm1, k.inv_gm1) + 0.5 * rho * (vx * vx + vy * vy);
 }
 
+template <bool ANY>
+__device__ __forceinline__ double gravity_factor(double s2)
+{
+    return ANY ? inv_pow15_rn(s2) : crm::pow_m15_rn(s2);
+}
+
 // cbdgam_2d.c:108-203: gravity, sink and their work on the gas for one mass,
-// given T = p / Sigma, the disk height h and gamma - 1 with its reciprocal
-template <class V>
+// given T = p / Sigma, the disk height h and gamma - 1 with its reciprocal.
+// FAR takes the short form beyond the sink's reach, where the stages lose
+// nothing by it: a term that is zero times a non-finite value adds a NaN to a
+// conserved value that already is one. ANY: any r^2 + softening^2 and T.
+template <bool FAR, bool ANY, class V>
 __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, double dt, const V &p, double T,
                                             double h, int constant_softening, double gm1, double inv_gm1, double *du,
                                             const double *g_in = nullptr, double *g_out = nullptr)
@@ -228,11 +237,11 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
     // Beyond four sink radii (with a margin far above the square root's
     // rounding) the sink rate is zero and the softening, if it follows the
     // disk height, is half of it: only gravity's terms are left, the others
-    // being exact zeros.
+    // being exact zeros for a finite state.
     const double far2 = 16.0 * (m.radius * m.radius);
-    if (r2 > far2 * (1.0 + 1e-10)) {
+    if (FAR && r2 > far2 * (1.0 + 1e-10)) {
         const double soft = constant_softening ? m.soft : 0.5 * h;
-        const double g = g_in ? *g_in : crm::pow_m15_rn(r2 + soft * soft);
+        const double g = g_in ? *g_in : gravity_factor<ANY>(r2 + soft * soft);
         if (g_out)
             *g_out = g;
         const double fnum = m.model >= 1 && m.model <= 3 ? sigma * m.mass * g : 0.0;
@@ -243,7 +252,7 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
         du[3] = dt * (fx * p[1] + fy * p[2]);
         return;
     }
-    const double eps = div_by(T, gm1, inv_gm1);
+    const double eps = ANY ? T / gm1 : div_by(T, gm1, inv_gm1);
     const double dr = sqrt_rn(r2);
     const double rs = m.radius;
     double soft;
@@ -258,7 +267,7 @@ __device__ __forceinline__ void mass_source(const Mass &m, double x, double y, d
     }
     const double rate = (dr < 4.0 * rs) ? m.rate * exp_rn(-fourth_rn(dr / rs)) : 0.0;
     // the gravity factor: from the face cache (constant softening), or computed
-    const double g = g_in ? *g_in : crm::pow_m15_rn(r2 + soft * soft);
+    const double g = g_in ? *g_in : gravity_factor<ANY>(r2 + soft * soft);
     if (g_out)
         *g_out = g;
     const double fnum = sigma * m.mass * g;
@@ -491,7 +500,7 @@ __global__ void source_kernel(int ni, int nj, double xl, double yl, double dx, d
         const double *p = prim + at(i, j, nj);
         const double T = p[3] / p[0];
         const double h = massless ? 1.0 : sqrt(T) / root_w2(ms, xc, yc);  // cbdgam_2d.c:75-106
-        mass_source(ms[which - 1], xc, yc, 1.0, p, T, h, constant_softening, gm1, inv_gm1, rate + at(i, j, nj));
+        mass_source<false, true>(ms[which - 1], xc, yc, 1.0, p, T, h, constant_softening, gm1, inv_gm1, rate + at(i, j, nj));
     }
 }
 
@@ -536,35 +545,38 @@ struct RedArgs {
 // a mass's source rates (dt = 1) for a diagnostic: the accretion rates
 // (masses zero) when its accretion flag is set, else the gravity rates
 // (sink rates zero), as the reference's reductions pass mass * gravity and
-// sink_rate * accretion (cbdgam_2d.py:104-139, 346-349, 397-402)
+// sink_rate * accretion (cbdgam_2d.py:104-139, 346-349, 397-402); the first
+// three, rate[3] is not used. ANY: a zone of any values, whose non-finite ones
+// show, else one that zone_in_range has passed.
+template <bool ANY>
 __device__ __forceinline__ void diag_rates(const RedArgs &r, const Diag &d, int which, double xc, double yc,
                                            const double *p, double *rate)
 {
     Mass m = r.m[which - 1];
-    const double T = p[3] / p[0];  // enters through the height alone
+    const double T = ANY ? p[3] / p[0] : div_rn(p[3], p[0]);
     double h = 1.0;
     if (d.accretion) {
-        // without masses every height is 1; beyond the sink's reach the rates are
-        // zeros (of Sigma and the velocity, so that a NaN still shows)
+        // without masses every height is 1; beyond the sink's reach the rates
+        // of finite values are zeros
         const double dx = xc - m.x, dy = yc - m.y;
-        if (dx * dx + dy * dy > 16.0 * (m.radius * m.radius) * (1.0 + 1e-10)) {
-            rate[0] = -(p[0] * 0.0);
-            rate[1] = rate[0] * p[1];
-            rate[2] = rate[0] * p[2];
-            rate[3] = 0.0;
+        if (!ANY && dx * dx + dy * dy > 16.0 * (m.radius * m.radius) * (1.0 + 1e-10)) {
+            rate[0] = rate[1] = rate[2] = 0.0;
             return;
         }
         m.mass = m.mass * 0.0;
     } else {
         m.rate = m.rate * 0.0;
-        // the height enters through a softening that follows it
+        // the height enters through a softening that follows it (cbdgam_2d.c:75-106)
         const bool massless = r.m[0].mass == 0.0 && r.m[1].mass == 0.0;
-        if (!r.k.constant_softening && !massless)
-            h = sqrt(T) / root_w2(r.m, xc, yc);  // cbdgam_2d.c:75-106
+        if (!r.k.constant_softening && !massless) {
+            const double w = root_w2(r.m, xc, yc);
+            h = ANY ? sqrt(T) / w : div_rn(sqrt_rn(T), w);
+        }
     }
-    mass_source(m, xc, yc, 1.0, p, T, h, r.k.constant_softening, r.k.gm1, r.k.inv_gm1, rate);
+    mass_source<!ANY, ANY>(m, xc, yc, 1.0, p, T, h, r.k.constant_softening, r.k.gm1, r.k.inv_gm1, rate);
 }
 
+template <bool ANY>
 __device__ __forceinline__ void diag_value(const RedArgs &r, const Diag &d, double x, double y, const double *p,
                                            double *re, double *im)
 {
@@ -590,7 +602,7 @@ __device__ __forceinline__ void diag_value(const RedArgs &r, const Diag &d, doub
         if (d.which_mass != 3 && d.which_mass != which)
             continue;
         double rate[NF];
-        diag_rates(r, d, which, x, y, p, rate);
+        diag_rates<ANY>(r, d, which, x, y, p, rate);
         for (int q = 0; q < 3; ++q)
             f[q] += rate[q];
     }
@@ -600,30 +612,58 @@ __device__ __forceinline__ void diag_value(const RedArgs &r, const Diag &d, doub
         *re = x * (f[2] * cut) - y * (f[1] * cut);
 }
 
-// per-block partial sums in a fixed tree order; the wavespeed maximum
-__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(RedArgs r, const double *prim, double *partials)
+// whether the straight-line operations cover a zone, given T = p / Sigma
+__device__ __forceinline__ bool zone_in_range(const double *p, double T)
 {
-    __shared__ double sm[RED_VALUES][RED_THREADS];
-    cbd::chain_begin();
+    const int vx = __double2hiint(p[1]) & 0x7ff00000, vy = __double2hiint(p[2]) & 0x7ff00000;
+    return thermal_in_range(p[3], T) & (max(vx, vy) != 0x7ff00000);
+}
+
+// The values of a thread's zones z0, z0 + step, ... into v; false when one of
+// them needs ANY.
+template <bool ANY>
+__device__ __forceinline__ bool add_zones(const RedArgs &r, const double *prim, long z0, long step, double *v)
+{
     const Consts &k = r.k;
-    double v[RED_VALUES];
+    const long n = (long)k.ni * k.nj;
+    bool ok = true;
     for (int q = 0; q < RED_VALUES; ++q)
         v[q] = 0.0;
-    const long n = (long)k.ni * k.nj;
-    const long step = (long)gridDim.x * RED_THREADS, z0 = blockIdx.x * (long)RED_THREADS + threadIdx.x;
     cbd::ZoneWalk w(z0, step, k.nj);
     for (long z = z0; z < n; z += step, w.next()) {
         const int i = w.i, j = w.j;
         const double *p = prim + at(i, j, k.nj);
-        v[0] = max_nan(v[0], zone_wavespeed(p, k.gamma));
+        const double T = ANY ? p[3] / p[0] : div_rn(p[3], p[0]);
+        v[0] = max_nan(v[0], max_wavespeed(p, ANY ? sqrt(T * k.gamma) : sqrt_rn(T * k.gamma)));
+        ok &= zone_in_range(p, T);
         const double x = k.xl + (i + 0.5) * k.dx, y = k.yl + (j + 0.5) * k.dy;
         for (int d = 0; d < r.nd; ++d) {
             double re, im;
-            diag_value(r, r.d[d], x, y, p, &re, &im);
+            diag_value<ANY>(r, r.d[d], x, y, p, &re, &im);
             v[1 + 2 * d] += re;
             v[2 + 2 * d] += im;
         }
     }
+    return ok;
+}
+
+__device__ __noinline__ void add_any_zones(const RedArgs &r, const double *prim, long z0, long step, double *v)
+{
+    add_zones<true>(r, prim, z0, step, v);
+}
+
+// Per-block partial sums in a fixed tree order; the wavespeed maximum. A
+// thread that met a value outside the straight-line operations' range (a flag
+// kept beside the sums; tested zone by zone it cost 5 %) takes its zones again.
+__global__ void __launch_bounds__(RED_THREADS) reduce_kernel(const __grid_constant__ RedArgs r, const double *prim,
+                                                             double *partials)
+{
+    __shared__ double sm[RED_VALUES][RED_THREADS];
+    cbd::chain_begin();
+    double v[RED_VALUES];
+    const long step = (long)gridDim.x * RED_THREADS, z0 = blockIdx.x * (long)RED_THREADS + threadIdx.x;
+    if (!add_zones<false>(r, prim, z0, step, v))
+        add_any_zones(r, prim, z0, step, v);
     for (int q = 0; q < RED_VALUES; ++q)
         sm[q][threadIdx.x] = v[q];
     __syncthreads();

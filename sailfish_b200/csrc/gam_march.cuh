@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(BJ, MINB) stage_kernel(const Consts k, const S
             for (int m = 0; m < 2; ++m) {
                 double du[NF];
                 const bool cached_g = ROLE == ROLE_READER && k.constant_softening;
-                mass_source(st.m[m], xc, yc, dt, z0, T0, hc0, k.constant_softening, k.gm1, k.inv_gm1, du,
-                            cached_g ? &gz[m] : nullptr, ROLE == ROLE_WRITER ? &gz[m] : nullptr);
+                mass_source<true, false>(st.m[m], xc, yc, dt, z0, T0, hc0, k.constant_softening, k.gm1, k.inv_gm1,
+                                         du, cached_g ? &gz[m] : nullptr, ROLE == ROLE_WRITER ? &gz[m] : nullptr);
 #pragma unroll
                 for (int q = 0; q < NF; ++q)
                     u[q] += du[q];

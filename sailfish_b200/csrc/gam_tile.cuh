@@ -225,7 +225,7 @@ __device__ __forceinline__ void tile_phase2(const Consts &k, const Stage &st, co
     for (int m = 0; m < 2; ++m) {
         double du[NF];
         const bool cached_g = ROLE == ROLE_READER && k.constant_softening;
-        mass_source(st.m[m], xc, yc, dt, c, T, hc, k.constant_softening, k.gm1, k.inv_gm1, du,
+        mass_source<true, false>(st.m[m], xc, yc, dt, c, T, hc, k.constant_softening, k.gm1, k.inv_gm1, du,
                     cached_g ? &gz[m] : nullptr, ROLE == ROLE_WRITER ? &gz[m] : nullptr);
 #pragma unroll
         for (int q = 0; q < NF; ++q)
