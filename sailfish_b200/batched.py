@@ -40,6 +40,12 @@ class Disk(NamedTuple):
     solution: Optional[np.ndarray] = None
 
 
+def default_tile(ni, nj):
+    """Tile shape (strip_width, rows) of a disk by its own size, for callers
+    that lay out `tiles` themselves (`default_tiles` goes by the whole batch)."""
+    return (128 if nj > 96 else 64), (32 if ni >= 512 else 16)
+
+
 # CTAs of the batched stage kernel resident at a time: 6 on each of 148 SMs
 _SMS, _SLOTS = 148, 148 * 6
 
@@ -61,7 +67,7 @@ def default_tiles(sizes):
     disks to 1024^2 361 / 464 / 360 / 468, 18 disks 577 / 594 / 560 / 594, 24
     disks 783 / 773 / 777 / 752, 35 disks 1240 / 1215 / 1218 / 1206.
     """
-    strips = {s: (128 if s[1] > 96 else 64) for s in sizes}
+    strips = {s: default_tile(*s)[0] for s in sizes}
 
     def tiles(rows):
         return sum(-(-nj // strips[ni, nj]) * -(-ni // rows) for ni, nj in sizes)
