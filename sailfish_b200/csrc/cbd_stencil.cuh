@@ -363,12 +363,16 @@ __device__ __forceinline__ void cons_to_prim(const double *u, double *p, const C
 }
 
 // max |v +- cs| over both directions, cbdiso_2d.c:340-350
-__device__ __forceinline__ double max_wavespeed(const double *p, double cs2)
+__device__ __forceinline__ double signal_speed(const double *p, double cs)
 {
-    const double cs = crm::sqrt_any(cs2);
     const double ax = greater(fabs(p[1] - cs), fabs(p[1] + cs));
     const double ay = greater(fabs(p[2] - cs), fabs(p[2] + cs));
     return greater(ax, ay);
+}
+
+__device__ __forceinline__ double max_wavespeed(const double *p, double cs2)
+{
+    return signal_speed(p, crm::sqrt_any(cs2));
 }
 
 // Source rates of both masses at the end-of-step time with dt = 1 and the

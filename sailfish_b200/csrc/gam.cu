@@ -485,22 +485,52 @@ __global__ void wavespeed_kernel(int ni, int nj, double gamma, const double *pri
     }
 }
 
-__global__ void source_kernel(int ni, int nj, double xl, double yl, double dx, double dy, Mass m1, Mass m2,
-                              int which, int constant_softening, double gm1, double inv_gm1, const double *prim,
-                              double *rate)
+// whether the straight-line operations cover a zone, given T = p / Sigma
+__device__ __forceinline__ bool zone_in_range(const double *p, double T)
 {
-    const Mass ms[2] = {m1, m2};
-    const bool massless = m1.mass == 0.0 && m2.mass == 0.0;
-    const long n = (long)ni * nj;
+    const int vx = __double2hiint(p[1]) & 0x7ff00000, vy = __double2hiint(p[2]) & 0x7ff00000;
+    return thermal_in_range(p[3], T) & (max(vx, vy) != 0x7ff00000);
+}
+
+struct SourceArgs {
+    int ni, nj;
+    double xl, yl, dx, dy;
+    Mass m[2];
+    int which, constant_softening, massless;
+    double gm1, inv_gm1;
+};
+
+// one zone's source terms; ANY as in mass_source, with the height by CUDA's operators
+template <bool ANY>
+__device__ __forceinline__ void zone_source(const SourceArgs &a, int i, int j, const double *p, double T, double *rate)
+{
+    const double xc = a.xl + (i + 0.5) * a.dx, yc = a.yl + (j + 0.5) * a.dy;
+    double h = 1.0;  // cbdgam_2d.c:75-106
+    if (!a.massless) {
+        const double w = root_w2(a.m, xc, yc);
+        h = ANY ? sqrt(T) / w : div_rn(sqrt_rn(T), w);
+    }
+    mass_source<!ANY, ANY>(a.m[a.which - 1], xc, yc, 1.0, p, T, h, a.constant_softening, a.gm1, a.inv_gm1, rate);
+}
+
+__device__ __noinline__ void any_zone_source(const SourceArgs &a, int i, int j, const double *p, double *rate)
+{
+    zone_source<true>(a, i, j, p, p[3] / p[0], rate);
+}
+
+__global__ void source_kernel(const __grid_constant__ SourceArgs a, const double *prim, double *rate)
+{
+    const long n = (long)a.ni * a.nj;
     const long step = (long)gridDim.x * blockDim.x, z0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    cbd::ZoneWalk w(z0, step, nj);
+    cbd::ZoneWalk w(z0, step, a.nj);
     for (long z = z0; z < n; z += step, w.next()) {
-        const int i = w.i, j = w.j;
-        const double xc = xl + (i + 0.5) * dx, yc = yl + (j + 0.5) * dy;
-        const double *p = prim + at(i, j, nj);
-        const double T = p[3] / p[0];
-        const double h = massless ? 1.0 : sqrt(T) / root_w2(ms, xc, yc);  // cbdgam_2d.c:75-106
-        mass_source<false, true>(ms[which - 1], xc, yc, 1.0, p, T, h, constant_softening, gm1, inv_gm1, rate + at(i, j, nj));
+        const double *p = prim + at(w.i, w.j, a.nj);
+        double *r = rate + at(w.i, w.j, a.nj);
+        const double T = div_rn(p[3], p[0]);
+        if (zone_in_range(p, T))
+            zone_source<false>(a, w.i, w.j, p, T, r);
+        else
+            any_zone_source(a, w.i, w.j, p, r);
     }
 }
 
@@ -610,13 +640,6 @@ __device__ __forceinline__ void diag_value(const RedArgs &r, const Diag &d, doub
         *re = f[0] * cut;
     else  // torque
         *re = x * (f[2] * cut) - y * (f[1] * cut);
-}
-
-// whether the straight-line operations cover a zone, given T = p / Sigma
-__device__ __forceinline__ bool zone_in_range(const double *p, double T)
-{
-    const int vx = __double2hiint(p[1]) & 0x7ff00000, vy = __double2hiint(p[2]) & 0x7ff00000;
-    return thermal_in_range(p[3], T) & (max(vx, vy) != 0x7ff00000);
 }
 
 // The values of a thread's zones z0, z0 + step, ... into v; false when one of
@@ -1046,12 +1069,21 @@ int cbdgam_2d_point_mass_source_term(int ni, int nj, double xl, double xr, doubl
 {
     if (ni <= 0 || nj <= 0 || !primitive || !cons_rate || (which_mass != 1 && which_mass != 2))
         return CBD_ERR_ARGUMENT;
-    const Mass m1 = mass_args(x1, y1, vx1, vy1, mass1, softening_length1, sink_rate1, sink_radius1, sink_model1);
-    const Mass m2 = mass_args(x2, y2, vx2, vy2, mass2, softening_length2, sink_rate2, sink_radius2, sink_model2);
-    source_kernel<<<blocks_for((long)ni * nj, 256), 256, 0,
-                    cbd::drop_in_stream()>>>(
-        ni, nj, xl, yl, (xr - xl) / ni, (yr - yl) / nj, m1, m2, which_mass, constant_softening, gamma_law_index - 1.0,
-        1.0 / (gamma_law_index - 1.0), primitive, cons_rate);
+    SourceArgs a;
+    a.ni = ni;
+    a.nj = nj;
+    a.xl = xl;
+    a.yl = yl;
+    a.dx = (xr - xl) / ni;
+    a.dy = (yr - yl) / nj;
+    a.m[0] = mass_args(x1, y1, vx1, vy1, mass1, softening_length1, sink_rate1, sink_radius1, sink_model1);
+    a.m[1] = mass_args(x2, y2, vx2, vy2, mass2, softening_length2, sink_rate2, sink_radius2, sink_model2);
+    a.which = which_mass;
+    a.constant_softening = constant_softening;
+    a.massless = mass1 == 0.0 && mass2 == 0.0;
+    a.gm1 = gamma_law_index - 1.0;
+    a.inv_gm1 = 1.0 / a.gm1;
+    source_kernel<<<blocks_for((long)ni * nj, 256), 256, 0, cbd::drop_in_stream()>>>(a, primitive, cons_rate);
     return status_of(cudaGetLastError());
 }
 

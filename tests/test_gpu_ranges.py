@@ -107,6 +107,23 @@ def test_isothermal_wavespeed_array(cs2):
     assert np.array_equal(ws.cpu().numpy()[2:-2, 2:-2], want)
 
 
+@pytest.mark.parametrize("mach2", [1e-150, 100.0, 1e150, 1e297, 1e305])
+def test_locally_isothermal_wavespeed_array(mach2):
+    from oracle import host as oh
+
+    p = _padded(np.ones((5, 7, 3)) * [1.0, 0.0, 0.0])
+    dp = torch.from_numpy(p).cuda()
+    ws = torch.zeros(dp.shape[:2], dtype=torch.float64, device="cuda")
+    m = [oh.Mass(0.5, x, 0.1, 0.0, 0.0, 0.05, 1, 1.0, 0.1) for x in (0.5, -0.5)]
+    want = np.zeros(p.shape[:2])
+    oh.Kernels("oracle", 1.5).wavespeed(5, 7, -1.0, 1.0, -1.0, 1.0, 0.0, mach2, 2, *m, p, want)
+    lib = _capi.lib()
+    lib.cbdiso_b200_set_stream(ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert lib.cbdiso_2d_wavespeed(5, 7, -1.0, 1.0, -1.0, 1.0, 0.0, mach2, 2, *m[0].args(), *m[1].args(), _ptr(dp),
+                                   _ptr(ws)) == 0
+    assert np.array_equal(ws.cpu().numpy(), want)
+
+
 def test_powers_outside_their_safe_range():
     x = np.array([1e-120, 1e-200, 1e120, 1e200, 0.0, np.inf, -0.5, -0.999, -1.0, -0.25])
     dx, out = torch.from_numpy(x).cuda(), torch.zeros(8 * x.size, dtype=torch.float64, device="cuda")
