@@ -630,8 +630,9 @@ void cbdgam_b200_abi_sizes(size_t out[2]);
 
 /* Test hook (no counterpart in the reference): the correctly rounded powers
  * the gamma-law kernels use, on device arrays of n elements: out[8i + 0..6]
- * = x^3, x^-2, x^-3, x^4, x^-1.5, (1 + x)^RN(-1/3), exp(-x), and in out[8i + 7]
- * r^-3 of the rounded root r of the rounded x^2 + 1e-12. */
+ * = x^3, x^-2, x^-3 (which no kernel uses any more), x^4, x^-1.5,
+ * (1 + x)^RN(-1/3), exp(-x), and in out[8i + 7] r^-3 of the rounded root r of
+ * the rounded x^2 + 1e-12. */
 int cbdgam_b200_eval_powers(long n, const double *x, double *out, void *stream);
 
 #ifdef __cplusplus

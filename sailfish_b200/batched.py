@@ -66,6 +66,9 @@ def default_tiles(sizes):
     16 rows everywhere / 16 and 32 / 8 and 16 / 8 and 32, from 512^2 on): 12
     disks to 1024^2 361 / 464 / 360 / 468, 18 disks 577 / 594 / 560 / 594, 24
     disks 783 / 773 / 777 / 752, 35 disks 1240 / 1215 / 1218 / 1206.
+    From 1.4 waves of 32-row tiles on those are the tall ones, and the smallest
+    disks that make up about 14 (with 16 rows 9) rows of strips per slot get the
+    short: lines drawn between those measurements, not derived.
     """
     strips = {s: default_tile(*s)[0] for s in sizes}
 

@@ -487,9 +487,10 @@ __device__ __forceinline__ void rho_strain_of(const Consts &k, double rho, const
 // Straight-line code (choices by selects), so that the march's two faces of a
 // row overlap in one thread.
 template <int DIR, class Acc>
-__device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, const double *pL, const double *pR, const double *gL, const double *gR,
-                                         const double *rL, const double *rR, const double *lul, const double *lur,
-                                         double xf, double yf, Acc &par, double *o)
+__device__ __forceinline__ void face_vjp(const Consts &k, const StageDev &st, const double *pL, const double *pR,
+                                         const double *gL, const double *gR, const double *rL, const double *rR,
+                                         const double *lul, const double *lur, double xf, double yf, Acc &par,
+                                         double *o)
 {
     const double hn = 0.5 * k.nu, b = st.one_minus_a;
     const double cf = b * st.dt * (DIR ? k.inv_dy : k.inv_dx);
@@ -622,8 +623,6 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) adj_faces(Consts 
     const int ni = k.ni, nj = k.nj;
     const long wi = ni + 2, wj = nj + 2, n = wi * wj;
     ParAcc<CHAIN> par(sh.jac);
-    MassT<double> m[2];
-    masses_t<double>(st, nullptr, m);
     const long f = grid_start(ADJ_THREADS);
     const bool ydir = f >= n;
     const long z = ydir ? f - n : f;
@@ -935,8 +934,6 @@ __global__ void __launch_bounds__(AM_NT, 3) adj_march(Consts k, AdjArgs a, int s
     load_stage<CHAIN>(a, sh);
     const StageDev &st = sh.st;
     ParAcc<CHAIN> par(sh.jac);
-    MassT<double> m[2];
-    masses_t<double>(st, nullptr, m);
 
     const int ni = k.ni, nj = k.nj, t = threadIdx.x;
     const int j0 = blockIdx.x * AM_BJ;

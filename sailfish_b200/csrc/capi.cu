@@ -171,10 +171,13 @@ namespace {
 // rule each time): 256^2 - / 33.0 / 33.9, 512^2 60.1 / 59.2 / 60.4, 768^2
 // 93.0 / 92.5 / 95.5, 900^2 133 / 135 / 143, 1024^2 147 / 158 / 158, 1200^2
 // 196 / 211 / 213, 1511^2 286 / 301 / 306, 2048^2 477 / 509 / 495, 3000^2 965 /
-// 975 / 1006; up to 128 columns, 128-column strips at 5 / 64 at 12: 16^2 23.3 /
-// 24.8, 64^2 25.8 / 27.1, 96^2 25.9 / 27.3. Long grids of at most 64 columns
-// keep 64-column strips (10 CTAs): 4096 x 64 66 against 72, 16384 x 64 175
-// against 211 (4096 x 32 60 against 56).
+// 975 / 1006. Just above a multiple of 256 columns the last strip idles and 128
+// columns at 5 CTAs are the better choice, which the rule does not make (256 /
+// 128 at 5): 1025^2 168 / 163, 1100^2 179 / 177, 1281^2 239 / 236, 2000 x 1300 359
+// / 338, 4096 x 1025 564 / 518, 2049^2 517 / 510. Up to 128 columns, 128-column
+// strips at 5 / 64 at 12: 16^2 23.3 / 24.8, 64^2 25.8 / 27.1, 96^2 25.9 / 27.3.
+// Long grids of at most 64 columns keep 64-column strips (10 CTAs): 4096 x 64 66
+// against 72, 16384 x 64 175 against 211 (4096 x 32 60 against 56).
 LaunchShape stage_shape(int ni, int nj, int bj, int rows, int occupancy = 0)
 {
     const bool chosen = rows <= 0;

@@ -69,7 +69,6 @@ struct Stage {
 using crm::cube_rn;
 using crm::exp_rn;
 using crm::fourth_rn;
-using crm::inv_cube_rn;
 using crm::inv_pow15_rn;
 using crm::inv_square_rn;
 using crm::pow_m13_rn;
@@ -722,6 +721,19 @@ __global__ void __launch_bounds__(32 * RED_VALUES) finish_kernel(const double *p
     }
     if (lane == 0)
         result[q] = s;
+}
+
+// RN(x^-3), the hook's alone (the kernels cube a root: inv_cube_of_sqrt_rn): x^3
+// as a double-double p + e, whose reciprocal's first approximation q = RN(1 / p)
+// leaves the exact residual 1 - q p, and one correction rounds once
+__device__ __forceinline__ double inv_cube_rn(double x)
+{
+    if (!crm::in_range(fabs(x)))
+        return pow(x, -3.0);
+    const double h = x * x, l = fma(x, x, -h);
+    const double p = h * x, e = fma(h, x, -p) + l * x;
+    const double q = 1.0 / p;
+    return q + q * (fma(-q, p, 1.0) - q * e);
 }
 
 // the correctly rounded helpers on device arrays (a test hook)

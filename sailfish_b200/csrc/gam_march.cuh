@@ -21,7 +21,7 @@
 //
 // What bounds it is the latency of a row's chain of dependent FP64 operations
 // at 12 warps per SM (168 registers; at 128 it spills 170 bytes and runs 8 %
-// slower): FP64 pipe 57 % busy, issue 0.56 per cycle, DRAM a tenth of its peak.
+// slower): FP64 pipe 57 % busy, issue 0.56 per cycle, DRAM a fifth of its peak.
 // Against the tiles of gam_tile.cuh it executes 756 instead of 835 FP64
 // instructions per zone in a reader stage (1041 against 1113 in a writer):
 // 2048^2 0.867 -> 0.752 ms per step, 1024^2 227 -> 206 us.
