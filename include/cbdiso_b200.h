@@ -125,7 +125,7 @@ typedef struct cbd_grid {
     double plm_theta;
     int eos_type;           /* 1 globally isothermal, 2 locally isothermal */
     int precision;          /* CBD_PRECISION_* */
-    double cs2;             /* sound_speed^2 (eos 1) */
+    double cs2;             /* sound_speed^2 (eos 1); zero, or within 2^-960 .. 2^960 for rounded face roots */
     double mach2;           /* mach_number^2 (eos 2) */
     double nu;              /* constant kinematic viscosity, 0 = inviscid */
     double velocity_ceiling;
