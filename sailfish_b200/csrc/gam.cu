@@ -152,7 +152,10 @@ __device__ __forceinline__ void buffer_source(const Consts &k, const Stage &st, 
         const double px = pf * div_by(-y, rc, yr), py = pf * div_by(x, rc, yr);
         const double ek = div_by(0.5 * (px * px + py * py), k.buf_sigma, k.inv_buf_sigma);
         const double target[NF] = {k.buf_sigma, px, py, k.buf_energy + ek};
-        const double rate = div_by(st.buf_k * (rc - k.buf_onset), k.buf_span, k.inv_buf_span);
+        // a ramp of no width, or one that starts at the origin, has an infinite
+        // rate, as in the reference
+        const double ramp = st.buf_k * (rc - k.buf_onset), steep = ramp * k.inv_buf_span;
+        const double rate = isinf(steep) ? steep : div_by(ramp, k.buf_span, k.inv_buf_span);
 #pragma unroll
         for (int q = 0; q < NF; ++q)
             u[q] -= (u[q] - target[q]) * rate * dt;
